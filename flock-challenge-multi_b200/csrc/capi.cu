@@ -52,6 +52,20 @@ std::atomic<uint64_t>& kernel_launch_counter() {
   return n;
 }
 
+const DeviceTimeouts& device_timeouts() {
+  static const DeviceTimeouts d = [] {
+    void *h = nullptr, *g = nullptr;
+    CK(cudaHostAlloc(&h, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable));
+    *static_cast<unsigned*>(h) = 0;
+    CK(cudaHostGetDevicePointer(&g, h, 0));
+    return DeviceTimeouts{static_cast<unsigned*>(h), static_cast<unsigned*>(g)};
+  }();
+  return d;
+}
+void check_device_timeouts() {
+  if (*device_timeouts().host) throw CudaError("a kernel's bounded wait ran out");
+}
+
 int resident_grid(const void* kernel, int threads, size_t smem, int sms) {
   static std::mutex mu;
   static std::map<std::tuple<const void*, int, size_t, int>, int> per_sm;
@@ -645,6 +659,7 @@ int flock_pcs_commit(flock_ctx* c, const uint64_t* z_packed, uint32_t m, uint8_t
     merkle_build(pd->cw, pd->n_leaves, 64 * sizeof(f128), pd->tree, c->st);
     CK(cudaMemcpyAsync(root32, pd->tree + 8 * (2 * pd->n_leaves - 2), 32, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    check_device_timeouts();
     *out = pd.release();
     return FLOCK_OK;
   });
@@ -1139,6 +1154,7 @@ int flock_ntt_rs_encode(flock_ctx* c, const uint64_t* msg, uint32_t log_msg_pos,
     ntt_rs_encode(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, c->st);
     CK(cudaMemcpyAsync(out, dc.p, nc * 16, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    check_device_timeouts();
     return FLOCK_OK;
   });
 }
@@ -1155,6 +1171,7 @@ int flock_ntt_rs_encode_plan(flock_ctx* c, const uint64_t* msg, uint32_t log_msg
     ntt_rs_encode_plan(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, plan_index, c->st);
     CK(cudaMemcpyAsync(out, dc.p, nc * 16, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    check_device_timeouts();
     return FLOCK_OK;
   });
 }

@@ -88,6 +88,16 @@ struct MpCoeffs {
   f128 c[8];
 };
 
+// A word of mapped host memory that kernels with bounded waits set when a wait
+// ran out; check_device_timeouts throws then (after a synchronisation of the
+// work it asks about).
+struct DeviceTimeouts {
+  volatile unsigned* host;
+  unsigned* dev;
+};
+const DeviceTimeouts& device_timeouts();
+void check_device_timeouts();
+
 // K0
 void launch_witness_seed(uint64_t seed, uint32_t log2, uint32_t n_blocks, uint32_t n_slots, f128* z, f128* a,
                          f128* b, cudaStream_t s);
@@ -131,7 +141,8 @@ struct NttPass {
   // 0: a thread owns a position pair and its lanes, products by integer
   // multiplies; 1: a warp owns a position pair's 64 lanes (lgs = 6) and
   // multiplies through a 4-bit window table of the warp-uniform twiddle;
-  // 2: as 1, with half of the lanes through the integer product
+  // 2: as 1, with half of the lanes through the integer product; 3: a CTA owns
+  // 64 lanes of its positions and multiplies on the tensor cores (forward only)
   int kind = 0;
 };
 using NttPlan = std::vector<NttPass>;
@@ -155,6 +166,7 @@ void ntt_transposed_encode(f128* e, f128* out, int log_msg, int log_inv_rate, cu
 // device-resident job table; every launch of the commit covers all jobs, a
 // thread block finding its job by binary search over the per-launch first
 // indices (jobs that take no part in a launch have an empty range).
+constexpr int kMaxBatchPasses = 6;
 struct BatchJob {
   uint64_t seed;  // witness inputs from the benchmark generator
   uint32_t log2, n_blocks, n_slots;
@@ -165,8 +177,10 @@ struct BatchJob {
   int log_d;
   uint64_t msg_len, rep0;  // message values; first element in the replicate launch
   int n_pass;
-  NttPass pass[4];
-  uint64_t tile0[4];  // first tile of this job in the launch of pass p
+  NttPass pass[kMaxBatchPasses];
+  // first tile of this job in the launch of pass p: of the tensor-core
+  // passes' launch for a kind-3 pass, of the other kinds' launch otherwise
+  uint64_t tile0[kMaxBatchPasses], tile0t[kMaxBatchPasses];
   uint32_t* tree;     // Merkle tree over 2^log_d leaves of 1 KiB
   uint64_t n_leaves, leaf0;
   uint64_t par0[24];  // first node of this job in the launch of parent level k
@@ -178,6 +192,9 @@ void ntt_replicate_batch(const BatchJob* jobs, int n_jobs, uint64_t total, cudaS
 size_t ntt_pass_batch_smem(const NttPass& p);
 void ntt_pass_batch(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_tiles, size_t smem, int grid,
                     cudaStream_t s);
+// the jobs' kind-3 passes; max_R: the largest layer count among them
+void ntt_pass_batch_t(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_tiles, int max_R, int sms,
+                      cudaStream_t s);
 void merkle_leaves_batch(const BatchJob* jobs, int n_jobs, uint64_t total, cudaStream_t s);
 void merkle_parents_batch(const BatchJob* jobs, int n_jobs, int level, uint64_t total, cudaStream_t s);
 void merkle_top_batch(const BatchJob* jobs, int n_jobs, cudaStream_t s);

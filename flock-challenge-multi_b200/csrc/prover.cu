@@ -217,9 +217,10 @@ BatchCommit batch_commit_async(const std::vector<Setup*>& setups, const std::vec
   if (n == 0) return h;
   if ((int)seeds.size() != n) throw std::runtime_error("batch_commit: one seed per setup");
   std::vector<BatchJob> J(n);
-  uint64_t wcta = 0, rep = 0, leaves = 0, tiles[4] = {0, 0, 0, 0}, par[24] = {0};
+  uint64_t wcta = 0, rep = 0, leaves = 0, par[24] = {0};
+  uint64_t tiles[kMaxBatchPasses] = {0}, tiles_t[kMaxBatchPasses] = {0};
   size_t smem = 0;
-  int max_pass = 0, max_level = 0;
+  int max_pass = 0, max_level = 0, max_R = 0;
   for (int i = 0; i < n; i++) {
     Setup& S = *setups[i];
     BatchJob& b = J[i];
@@ -238,15 +239,18 @@ BatchCommit batch_commit_async(const std::vector<Setup*>& setups, const std::vec
     b.rep0 = rep;
     rep += b.msg_len;
     const NttPlan plan = ntt_plan(b.log_d, 64, 1);
-    if (plan.size() > 4) throw std::runtime_error("batch_commit: more than four NTT passes");
+    if (plan.size() > kMaxBatchPasses) throw std::runtime_error("batch_commit: too many NTT passes");
     b.n_pass = (int)plan.size();
     max_pass = std::max(max_pass, b.n_pass);
-    for (int p = 0; p < 4; p++) {
+    for (int p = 0; p < kMaxBatchPasses; p++) {
       b.tile0[p] = tiles[p];
+      b.tile0t[p] = tiles_t[p];
       if (p < b.n_pass) {
         b.pass[p] = plan[p];
-        tiles[p] += ((uint64_t)1 << (b.log_d - plan[p].R)) * (uint64_t)(64 >> plan[p].lgs);
-        smem = std::max(smem, ntt_pass_batch_smem(plan[p]));
+        const bool tensor = plan[p].kind == 3;
+        (tensor ? tiles_t : tiles)[p] += ((uint64_t)1 << (b.log_d - plan[p].R)) * (uint64_t)(64 >> plan[p].lgs);
+        if (tensor) max_R = std::max(max_R, plan[p].R);
+        else smem = std::max(smem, ntt_pass_batch_smem(plan[p]));
       }
     }
     b.tree = S.tree0;
@@ -284,7 +288,10 @@ BatchCommit batch_commit_async(const std::vector<Setup*>& setups, const std::vec
     cudaGraphExec_t g = capture(st, &launches, [&] {
       launch_witness_seed_batch(dj, n, (uint32_t)wcta, st);
       // pass 0 reads each job's message as its replicated codeword
-      for (int p = 0; p < max_pass; p++) ntt_pass_batch(dj, n, p, tiles[p], smem, 2 * sms, st);
+      for (int p = 0; p < max_pass; p++) {
+        if (tiles[p]) ntt_pass_batch(dj, n, p, tiles[p], smem, 2 * sms, st);
+        if (tiles_t[p]) ntt_pass_batch_t(dj, n, p, tiles_t[p], max_R, sms, st);
+      }
       merkle_leaves_batch(dj, n, leaves, st);
       for (int l = 1; l <= max_level; l++) merkle_parents_batch(dj, n, l, par[l], st);
       merkle_top_batch(dj, n, st);
@@ -1129,6 +1136,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   }
   mark(9);
   CK(cudaStreamSynchronize(st));
+  check_device_timeouts();
   finish_openings();
   std::vector<uint8_t> bytes = encode(P);
   return bytes;
