@@ -966,9 +966,11 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     CK(cudaMemcpyAsync(bc_tabs, T.data(), T.size() * sizeof(f128), cudaMemcpyHostToDevice, st));
     // eq(suffix_k, i) = lo_k(i mod 2^lo_bits) * hi_k(i >> lo_bits), both tables
     // on the device; chunks of up to 2^14 values (each CTA builds its two
-    // product tables once per chunk), as long as the four tables fit eqbuf
+    // product tables once per chunk), as long as the four tables fit eqbuf,
+    // and 2^9 chunks if they leave 2^9 values each: with 2^14 a 2^10-compression
+    // proof had 8 chunks, 8 CTAs and 140 us here
     const int n_vars = (int)x_ab.size() - 1;
-    int lo_bits = std::min(n_vars, 14);
+    int lo_bits = std::min(n_vars, std::min(14, std::max(9, n_vars - 9)));
     while (lo_bits > 0 && 2 * ((1ull << lo_bits) + (1ull << (n_vars - lo_bits))) > n_words) lo_bits--;
     const int hi_bits = n_vars - lo_bits;
     f128* d = eqbuf[0];  // [lo0 | hi0 | lo1 | hi1]

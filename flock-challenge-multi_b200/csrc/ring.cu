@@ -84,15 +84,18 @@ __global__ void __launch_bounds__(256, 3) k_bcombined_msg(const f128* __restrict
                                                           f128* __restrict__ out, f128* __restrict__ msg) {
   extern __shared__ __align__(16) uint8_t sm[];
   Tab4* C = reinterpret_cast<Tab4*>(sm);
+  __shared__ f128 img[256];
   const size_t half = (size_t)1 << (lo_bits - 1);
   u256 u0 = zero256(), u2 = zero256();
   for (size_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
-    if (threadIdx.x < 64) {
-      const int k = threadIdx.x >> 5, w = threadIdx.x & 31;
-      const f128* L = k ? L1 : L0;
-      const f128 y = mul_x128(ldg((k ? ehi1 : ehi0) + ch), 4 * w);
-      tab4_window(C + k, w, apply_tab(L, y), apply_tab(L, mul_xk(y, 1)), apply_tab(L, mul_xk(y, 2)),
-                  apply_tab(L, mul_xk(y, 3)));
+    {  // thread (k, w, i): the image of basis vector 4 w + i under claim k's map
+      const int k = threadIdx.x >> 7, v = threadIdx.x & 127;
+      img[threadIdx.x] = apply_tab(k ? L1 : L0, mul_x128(ldg((k ? ehi1 : ehi0) + ch), v));
+    }
+    __syncthreads();
+    if (threadIdx.x < 64) {  // thread (k, w): window w of claim k's map
+      const f128* b = img + 4 * threadIdx.x;
+      tab4_window(C + (threadIdx.x >> 5), threadIdx.x & 31, b[0], b[1], b[2], b[3]);
     }
     __syncthreads();
     for (size_t j = threadIdx.x; j < half; j += blockDim.x) {

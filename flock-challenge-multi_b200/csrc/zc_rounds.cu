@@ -28,6 +28,11 @@
 // 2^nm pairs with shifts, multiplies once by etab[group], and keeps the
 // result per js.  The products by phi8(g(js)) and by the round's constant
 // factor are left to the host: out[2 js] = T1(js), out[2 js + 1] = Tinf(js).
+//
+// A lane that sums all 2^nm pairs of a group pays for the group's weight once,
+// but leaves most of the chip idle when there are few groups (8 CTAs at round 2
+// of a 2^10-compression proof: 78 us).  So a group's pairs are spread over
+// 2^(nm - nl) lanes, nl chosen by the launch so that the lanes fill one wave.
 #include "kernels.cuh"
 
 namespace {
@@ -38,8 +43,9 @@ struct ZcArgs {
   f128* b_out;
   const f128* lag;  // 8 x 256 Lagrange byte table (packed input)
   f128 rho;
-  size_t n_pairs;   // pairs of the message round
+  uint32_t n_pairs;  // pairs of the message round
   int ns, nm, msh;
+  int nl;  // a lane sums 2^nl of its group's 2^nm medium values
   const f128* etab;  // eq over the random suffix, indexed by group
   f128* out;
   f128* halve_out;   // next round's table: etab with its lowest variable summed out
@@ -71,7 +77,9 @@ __device__ __forceinline__ void xshfl(f128& v, int m) {
   v.hi ^= shfl_xor64(v.hi, m);
 }
 
-// MODE 0: packed message round; 1: packed fold + message; 2: fold + message
+// MODE 0: packed message round; 1: packed fold + message; 2: fold + message,
+// the fold through a window table of rho; 3: the same through plain products
+// (short rounds, where building the table takes longer than the folds)
 template <int MODE>
 __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
   extern __shared__ __align__(16) uint8_t smraw[];
@@ -84,26 +92,29 @@ __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
       if (MODE == 1) st(lag + 2048 + i, fmul(A.rho, v));
     }
     __syncthreads();
-  } else {
+  } else if (MODE == 2) {
     multab_build(rt, A.rho);
   }
+  auto fold = [&](f128 lo, f128 hi) {
+    const f128 d = fx(lo, hi);
+    return fx(lo, MODE == 2 ? multab_mul(rt, d) : fmul(A.rho, d));
+  };
   for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < A.halve_n; j += (size_t)gridDim.x * blockDim.x)
     st(A.halve_out + j, fx(ldg(A.etab + 2 * j), ldg(A.etab + 2 * j + 1)));
   const int lane = threadIdx.x & 31;
-  const int ns = A.ns, nm = A.nm, gb = ns + nm;
-  const int js = lane & ((1 << ns) - 1), gw = lane >> ns;
-  const size_t gpw = (size_t)32 >> ns;  // groups per warp iteration
-  const size_t n_groups = (A.n_pairs + ((size_t)1 << gb) - 1) >> gb;
-  const size_t warp0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const size_t n_warps = ((size_t)gridDim.x * blockDim.x) >> 5;
+  const int ns = A.ns, nm = A.nm, gb = ns + nm, nl = A.nl;
+  const int js = lane & ((1 << ns) - 1);
+  const uint32_t n_pairs = A.n_pairs;
+  const uint32_t n_items = ((n_pairs + (1u << gb) - 1) >> gb) << (gb - nl);
   f128 T1 = mk(0, 0), Ti = mk(0, 0);
-  for (size_t it = warp0; it * gpw < n_groups; it += n_warps) {
-    const size_t grp = it * gpw + gw;
-    if (grp >= n_groups) continue;
+  // item: (group, part of its medium values, js)
+  for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item < n_items; item += gridDim.x * blockDim.x) {
+    const uint32_t grp = item >> (gb - nl);
+    const int jm0 = (int)((item >> ns) & ((1u << (nm - nl)) - 1)) << nl;
     W3 s1 = {0, 0, 0}, si = {0, 0, 0};
-    for (int jm = 0; jm < (1 << nm); jm++) {
-      const size_t j = (grp << gb) | ((size_t)jm << ns) | (size_t)js;
-      if (j >= A.n_pairs) continue;  // short final rounds
+    for (int jm = jm0; jm < jm0 + (1 << nl); jm++) {
+      const uint32_t j = (grp << gb) | (uint32_t)(jm << ns) | (uint32_t)js;
+      if (j >= n_pairs) continue;  // short final rounds
       f128 a1, ad, b1, bd;           // x^(2j+1) and the pair sum
       if (MODE == 0) {
         const f128 wa = ldg(A.a_in + j), wb = ldg(A.b_in + j);
@@ -114,16 +125,16 @@ __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
       } else {
         f128 a0, b0;
         if (MODE == 1) {
-          const f128 w0 = ldg(A.a_in + 2 * j), w1 = ldg(A.a_in + 2 * j + 1);
-          const f128 v0 = ldg(A.b_in + 2 * j), v1 = ldg(A.b_in + 2 * j + 1);
+          const f128 w0 = ldg(A.a_in + 2 * (size_t)j), w1 = ldg(A.a_in + 2 * (size_t)j + 1);
+          const f128 v0 = ldg(A.b_in + 2 * (size_t)j), v1 = ldg(A.b_in + 2 * (size_t)j + 1);
           const f128* rl = lag + 2048;
           a0 = fx(lag_lookup(lag, w0.lo), lag_lookup(rl, w0.lo ^ w0.hi));
           a1 = fx(lag_lookup(lag, w1.lo), lag_lookup(rl, w1.lo ^ w1.hi));
           b0 = fx(lag_lookup(lag, v0.lo), lag_lookup(rl, v0.lo ^ v0.hi));
           b1 = fx(lag_lookup(lag, v1.lo), lag_lookup(rl, v1.lo ^ v1.hi));
         } else {
-          const ulonglong2* pa = reinterpret_cast<const ulonglong2*>(A.a_in + 4 * j);
-          const ulonglong2* pb = reinterpret_cast<const ulonglong2*>(A.b_in + 4 * j);
+          const ulonglong2* pa = reinterpret_cast<const ulonglong2*>(A.a_in + 4 * (size_t)j);
+          const ulonglong2* pb = reinterpret_cast<const ulonglong2*>(A.b_in + 4 * (size_t)j);
           f128 av[4], bv[4];
 #pragma unroll
           for (int k = 0; k < 4; k++) {
@@ -131,15 +142,15 @@ __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
             av[k] = mk(x.x, x.y);
             bv[k] = mk(y.x, y.y);
           }
-          a0 = fx(av[0], multab_mul(rt, fx(av[0], av[1])));
-          a1 = fx(av[2], multab_mul(rt, fx(av[2], av[3])));
-          b0 = fx(bv[0], multab_mul(rt, fx(bv[0], bv[1])));
-          b1 = fx(bv[2], multab_mul(rt, fx(bv[2], bv[3])));
+          a0 = fold(av[0], av[1]);
+          a1 = fold(av[2], av[3]);
+          b0 = fold(bv[0], bv[1]);
+          b1 = fold(bv[2], bv[3]);
         }
-        st(A.a_out + 2 * j, a0);
-        st(A.a_out + 2 * j + 1, a1);
-        st(A.b_out + 2 * j, b0);
-        st(A.b_out + 2 * j + 1, b1);
+        st(A.a_out + 2 * (size_t)j, a0);
+        st(A.a_out + 2 * (size_t)j + 1, a1);
+        st(A.b_out + 2 * (size_t)j, b0);
+        st(A.b_out + 2 * (size_t)j + 1, b1);
         ad = fx(a0, a1);
         bd = fx(b0, b1);
       }
@@ -181,20 +192,31 @@ void zc_round(int mode, const f128* a_in, const f128* b_in, f128* a_out, f128* b
               f128* halve_out, size_t halve_n) {
   if (ns < 0 || ns > 2 || nm < 0 || nm > 4 || msh < 0 || (nm > 0 && (((1 << nm) - 1) << msh) >= 64))
     throw CudaError("zc_round: bad eq structure");
+  if (n_pairs > ((size_t)1 << 30)) throw CudaError("zc_round: too many pairs");
   ZcArgs A;
   A.a_in = a_in; A.b_in = b_in; A.a_out = a_out; A.b_out = b_out; A.lag = lag; A.rho = rho;
-  A.n_pairs = n_pairs; A.ns = ns; A.nm = nm; A.msh = msh;
+  A.n_pairs = (uint32_t)n_pairs; A.ns = ns; A.nm = nm; A.msh = msh;
   A.etab = etab; A.out = out;
   A.halve_out = halve_out; A.halve_n = halve_n;
-  const size_t smem = mode == 0 ? 2048 * sizeof(f128) : mode == 1 ? 4096 * sizeof(f128) : sizeof(MulTab8);
-  const size_t lanes = (n_pairs + ((size_t)1 << nm) - 1) >> nm;
-  const void* fn = mode == 0 ? (const void*)k_zc_round<0> : mode == 1 ? (const void*)k_zc_round<1>
-                                                                      : (const void*)k_zc_round<2>;
-  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const size_t full = (size_t)resident_grid(fn, 256, smem, sms);
+  // the window table pays from about 2^14 folded pairs on (k_lig_fold_msg's line too)
+  const bool plain = mode == 2 && n_pairs < ((size_t)1 << 14);
+  const size_t smem = mode == 0 ? 2048 * sizeof(f128) : mode == 1 ? 4096 * sizeof(f128) : plain ? 0 : sizeof(MulTab8);
+  auto* fn = mode == 0 ? k_zc_round<0> : mode == 1 ? k_zc_round<1> : plain ? k_zc_round<3> : k_zc_round<2>;
+  if (smem) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const size_t full = (size_t)resident_grid((const void*)fn, 256, smem, sms);
+  // passes of the wave over the items, each 2^nl pairs (two products and the
+  // folds) and one weighting (two products)
+  size_t best = ~(size_t)0;
+  for (int nl = nm; nl >= 0; nl--) {
+    const size_t items = std::max<size_t>(1, n_pairs >> nl);
+    const size_t cost = (items + full * 256 - 1) / (full * 256) * (((size_t)2 << nl) + 1);
+    if (cost < best) {
+      best = cost;
+      A.nl = nl;
+    }
+  }
+  const size_t lanes = n_pairs >> A.nl;
   const int g = (int)std::max<size_t>(1, std::min<size_t>(full, (lanes + 255) / 256));
   count_launch();
-  if (mode == 0) k_zc_round<0><<<g, 256, smem, s>>>(A);
-  else if (mode == 1) k_zc_round<1><<<g, 256, smem, s>>>(A);
-  else k_zc_round<2><<<g, 256, smem, s>>>(A);
+  fn<<<g, 256, smem, s>>>(A);
 }
