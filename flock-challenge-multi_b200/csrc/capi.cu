@@ -1443,23 +1443,15 @@ int flock_bench_sumcheck3(flock_ctx* c, size_t n, int iters, double* ms) {
 
 // ---- degree-4 zerocheck round 1 (zerocheck/univariate_skip_deg4.rs)
 namespace {
-// eq(r, .) over n <= 30 variables on the device, low variables first
-void eq_device(const f128* r, int n, f128* lo, f128* hi, f128* out, cudaStream_t st) {
-  const int s = std::min(n, 12);
-  eq_build(r, s, flock::hone(), lo, st);
-  eq_build(r + s, n - s, flock::hone(), hi, st);
-  eq_split(lo, hi, s, (size_t)1 << n, out, st);
-}
 struct Deg4Bufs {
   size_t rows;
   DevBuf<uint64_t> v;  // a, b, c, d, z rows
-  DevBuf<f128> eq, lo, hi, sums;  // sums: H (1536) then Zs (64)
+  DevBuf<f128> eq, sums;  // sums: H (1536) then Zs (64)
   DevBuf<uint8_t> tab;
   explicit Deg4Bufs(uint32_t m)
-      : rows((size_t)1 << (m - 6)), v(5 * rows), eq(rows), lo(1 << 12), hi(std::max<size_t>(1, rows >> 12)),
-        sums(1600), tab(deg4_tables_bytes()) {}
+      : rows((size_t)1 << (m - 6)), v(5 * rows), eq(rows), sums(1600), tab(deg4_tables_bytes()) {}
   void run(const std::vector<f128>& r, int m, int sms, cudaStream_t st) {
-    eq_device(r.data() + 6, m - 6, lo.p, hi.p, eq.p, st);
+    eq_build(r.data() + 6, m - 6, flock::hone(), eq.p, st);
     CK(cudaMemsetAsync(sums.p, 0, 1600 * sizeof(f128), st));
     round1_deg4(v.p, v.p + rows, v.p + 2 * rows, v.p + 3 * rows, v.p + 4 * rows, eq.p, rows, tab.p, sums.p,
                 sums.p + 1536, 2 * sms, st);

@@ -217,8 +217,16 @@ __global__ void k_gather_rows(const f128* cw, const uint64_t* pos, size_t n, int
 uint64_t pow_search(const uint8_t digest[32], uint32_t bits, cudaStream_t s, unsigned long long* d_found,
                     unsigned long long* h_found, int fn = 1);
 // K3..K8
-void eq_split(const f128* lo, const f128* hi, int s_bits, size_t n, f128* out, cudaStream_t s);
 void axpy(f128* out, const f128* x, f128 beta, size_t n, cudaStream_t s);
+// eq tables out[i] = scale * prod_j (bit j of i ? r_j : 1 + r_j), i < 2^n, n <= 31
+struct EqTable {
+  const f128* r;  // host
+  int n;
+  f128 scale;
+  f128* out;
+};
+constexpr int kMaxEqTables = 4;
+void eq_build(const EqTable* tabs, int count, cudaStream_t s);  // one launch
 void eq_build(const f128* r, int n, f128 scale, f128* out, cudaStream_t s);
 void outer64(const f128* L, const f128* e, size_t n_e, f128* out, cudaStream_t s);
 void inner(const f128* f, const f128* g, size_t n, f128* out, int grid, cudaStream_t s);

@@ -108,8 +108,6 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   out = dalloc<f128>(1024, st);
   tabs_r1 = dalloc<uint8_t>(round1_tables_size(), st);
   lag = dalloc<f128>(8 * 256, st);
-  elo = dalloc<f128>(1 << 13, st);
-  ehi = dalloc<f128>(1 << 16, st);
   const size_t kk = (size_t)1 << k_log;
   comb = dalloc<f128>(kk, st);
   zv = dalloc<f128>(kk, st);
@@ -327,7 +325,7 @@ void batch_commit(const std::vector<Setup*>& setups, const std::vector<uint64_t>
 Setup::~Setup() {
   cudaStreamSynchronize(st);
   void* ptrs[] = {z, a, b, cw0, tree0, pp[0], pp[1], pp[2], pp[3], eqbuf[0], zv_pre, induce_buf, out, blocks_buf, records_buf,
-                  tabs_r1, lag, elo, ehi, comb, zv, eq_inner, bc_tabs, idx, gather, d_found, at_ptr, bt_ptr,
+                  tabs_r1, lag, comb, zv, eq_inner, bc_tabs, idx, gather, d_found, at_ptr, bt_ptr,
                   at_row, bt_row, kc_w};
   for (void* p : ptrs)
     if (p) cudaFreeAsync(p, st);
@@ -375,14 +373,8 @@ void Setup::build_round1_tables() {
   CK(cudaMemcpy(tabs_r1, host.data(), host.size(), cudaMemcpyHostToDevice));
 }
 
-// eq table of r into dev (length 2^|r|), as lo (<= 12 vars) x hi on the device
-void Setup::eq_table(const std::vector<f128>& r, f128* dev) {
-  size_t n = r.size();
-  int s = (int)std::min<size_t>(n, 12);
-  eq_build(r.data(), s, hone(), elo, st);
-  eq_build(r.data() + s, (int)n - s, hone(), ehi, st);
-  eq_split(elo, ehi, s, (size_t)1 << n, dev, st);
-}
+// eq table of r into dev (length 2^|r|)
+void Setup::eq_table(const std::vector<f128>& r, f128* dev) { eq_build(r.data(), (int)r.size(), hone(), dev, st); }
 
 void Setup::fetch(const f128* dev, size_t n, f128* host) {
   CK(cudaMemcpyAsync(host, dev, n * sizeof(f128), cudaMemcpyDeviceToHost, st));
@@ -536,10 +528,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     f128 C = hone();
     for (f128 bm : med) C = hmul(C, fx(hone(), bm));
     std::vector<f128> rh(r.begin() + 13, r.end());
-    int s = (int)std::min<size_t>(rh.size(), 12);
-    eq_build(rh.data(), s, hone(), elo, st);
-    eq_build(rh.data() + s, (int)rh.size() - s, C, ehi, st);
-    eq_split(elo, ehi, s, (size_t)1 << rh.size(), scratch_eq(), st);
+    eq_build(rh.data(), (int)rh.size(), C, scratch_eq(), st);
     CK(cudaMemsetAsync(out, 0, 1024 * sizeof(f128), st));
     size_t n_blocks128 = (size_t)1 << (m - 13);
     zc_round1(a, b, z, tabs_r1, scratch_eq(), n_blocks128, out, gs, st);
@@ -975,12 +964,14 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     const int hi_bits = n_vars - lo_bits;
     f128* d = eqbuf[0];  // [lo0 | hi0 | lo1 | hi1]
     const size_t nlo = (size_t)1 << lo_bits, nhi = (size_t)1 << hi_bits;
+    EqTable et[4];
     for (int k = 0; k < 2; k++) {
       const std::vector<f128>& xf = k == 0 ? x_ab : x_c;
       f128* base = d + k * (nlo + nhi);
-      eq_build(xf.data() + 1, lo_bits, hone(), base, st);
-      eq_build(xf.data() + 1 + lo_bits, hi_bits, hone(), base + nlo, st);
+      et[2 * k] = {xf.data() + 1, lo_bits, hone(), base};
+      et[2 * k + 1] = {xf.data() + 1 + lo_bits, hi_bits, hone(), base + nlo};
     }
+    eq_build(et, 4, st);
     // with no packed-direct claim, b_combined is final here: the first
     // Ligerito message (over z and b_combined) is summed in the same pass
     if (!chain && !merkle && lo_bits >= 1) first_msg = next_out(1);

@@ -192,7 +192,7 @@ class Setup {
   f128* pp[4] = {nullptr, nullptr, nullptr, nullptr};
   f128* eqbuf[2] = {nullptr, nullptr};
   std::vector<Level> levels;
-  f128 *induce_buf = nullptr, *out = nullptr, *lag = nullptr, *elo = nullptr, *ehi = nullptr;
+  f128 *induce_buf = nullptr, *out = nullptr, *lag = nullptr;
   f128 *comb = nullptr, *zv = nullptr, *zv_pre = nullptr, *eq_inner = nullptr, *bc_tabs = nullptr, *gather = nullptr;
   std::vector<f128> s_hat_v_c;  // c-claim ring-switch statistic, captured by zerocheck round 1
   uint8_t* tabs_r1 = nullptr;

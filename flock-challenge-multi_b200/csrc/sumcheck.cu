@@ -32,27 +32,53 @@ namespace {
 }  // namespace
 
 // ------------------------------------------------------------------ K3 --
-__global__ void k_eq_split(const f128* __restrict__ lo, const f128* __restrict__ hi, int s, size_t n,
-                           f128* __restrict__ out) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  st(out + i, fmul(ldg(lo + (i & ((1ull << s) - 1))), ldg(hi + (i >> s))));
-}
-
 // eq tables built on the device: out[i] = scale * prod_j (bit j of i ? r_j : 1 + r_j)
 // (the same values as the doubling construction of eq(r, .), field products
-// being exact)
+// being exact).  A table's cost is the chain of dependent products, about a
+// microsecond each, so the chain is kept short: a CTA tabulates variables 0..3
+// and 4..7, the next q, and multiplies the rest (its own index bits) in a
+// shuffle tree, all at once; an output then takes one product.
+// Up to 4 tables a launch (grid y).  Tables of up to 2^18 values take 7 us, one
+// of 2^19 40 us; one chain of up to 13 products per thread, and a third launch
+// for the tables above 2^12, took 18 + 18 + 4 us (54 us at 2^19).
 struct EqVec {
-  f128 r[24];
+  f128 r[32];
   f128 scale;
-  int n;
+  f128* out;
+  int n, q;
 };
-__global__ void k_eq_build(EqVec E, f128* __restrict__ out) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ((size_t)1 << E.n)) return;
-  f128 v = E.scale;
-  for (int j = 0; j < E.n; j++) v = fmul(v, ((i >> j) & 1) ? E.r[j] : fx(E.r[j], mk(1, 0)));
-  st(out + i, v);
+struct EqVecs {
+  EqVec v[kMaxEqTables];
+};
+__global__ void __launch_bounds__(256) k_eq_build(const __grid_constant__ EqVecs V) {
+  const EqVec& E = V.v[blockIdx.y];
+  const int n = E.n, q = E.q, t = threadIdx.x;
+  if (((uint64_t)blockIdx.x << (8 + q)) >> n) return;
+  __shared__ f128 T[3][16], H, K[16];
+  auto factor = [&](int j, uint32_t bit) { return j < n ? (bit ? E.r[j] : fx(E.r[j], mk(1, 0))) : mk(1, 0); };
+  if (t < 48) {  // entry e of the table of variables j0..j0+3
+    const int w = t >> 4, e = t & 15, j0 = 4 * w, nv = w < 2 ? 4 : q;
+    f128 v = nv ? factor(j0, e & 1) : mk(1, 0);
+    for (int j = 1; j < nv; j++) v = fmul(v, factor(j0 + j, (e >> j) & 1));
+    T[w][e] = v;
+  } else if (t >= 64 && t < 96) {  // the CTA's own index bits, and the scale
+    const int l = t - 64, own = max(n - 8 - q, 0);
+    f128 v = l < own ? factor(8 + q + l, (blockIdx.x >> l) & 1) : l == own ? E.scale : mk(1, 0);
+    for (int m = 1; m <= own; m <<= 1) {  // lane 0 collects lanes 0..2m-1
+      f128 o;
+      o.lo = shfl_xor64(v.lo, m);
+      o.hi = shfl_xor64(v.hi, m);
+      v = fmul(v, o);
+    }
+    if (l == 0) H = v;
+  }
+  __syncthreads();
+  const f128 lo = fmul(T[0][t & 15], T[1][t >> 4]);
+  if (t < (1 << q)) K[t] = fmul(T[2][t], H);
+  __syncthreads();
+  if (n < 8 && (t >> n)) return;
+  f128* out = E.out + ((size_t)blockIdx.x << (8 + q)) + t;
+  for (int k = 0; k < (1 << q); k++) st(out + ((size_t)k << 8), fmul(lo, K[k]));
 }
 
 // out[s + 64 k] = L[s] * e[k]
@@ -363,18 +389,28 @@ void lig_fold_msg(const f128* f, const f128* b, f128* fo, f128* bo, f128 r, size
     k_lig_fold_msg<false><<<grid, 256, 0, s>>>(f, b, fo, bo, r, n_pairs_out, emit, out);
   }
 }
-void eq_split(const f128* lo, const f128* hi, int s_bits, size_t n, f128* out, cudaStream_t s) {
-  count_launch(); k_eq_split<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(lo, hi, s_bits, n, out);
+void eq_build(const EqTable* tabs, int count, cudaStream_t s) {
+  if (count < 1 || count > kMaxEqTables) throw CudaError("eq_build: one to four tables");
+  EqVecs V;
+  unsigned blocks = 1;
+  for (int i = 0; i < count; i++) {
+    const EqTable& t = tabs[i];
+    if (t.n < 0 || t.n > 31) throw CudaError("eq_build: at most 31 variables");
+    EqVec& E = V.v[i];
+    for (int j = 0; j < t.n; j++) E.r[j] = t.r[j];
+    E.scale = t.scale;
+    E.out = t.out;
+    E.n = t.n;
+    // values per CTA 2^(8 + q): 2^10 CTAs before they grow
+    E.q = std::min(4, std::max(0, t.n - 18));
+    blocks = std::max(blocks, 1u << std::max(0, t.n - 8 - E.q));
+  }
+  count_launch();
+  k_eq_build<<<dim3(blocks, count), 256, 0, s>>>(V);
 }
 void eq_build(const f128* r, int n, f128 scale, f128* out, cudaStream_t s) {
-  if (n < 0 || n > 24) throw CudaError("eq_build: at most 24 variables");
-  EqVec E;
-  for (int j = 0; j < n; j++) E.r[j] = r[j];
-  E.scale = scale;
-  E.n = n;
-  const size_t len = (size_t)1 << n;
-  count_launch();
-  k_eq_build<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(E, out);
+  const EqTable t{r, n, scale, out};
+  eq_build(&t, 1, s);
 }
 void outer64(const f128* L, const f128* e, size_t n_e, f128* out, cudaStream_t s) {
   Vec64 V;
