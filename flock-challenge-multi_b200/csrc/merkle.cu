@@ -11,6 +11,8 @@
 #include "kernels.cuh"
 #include "sha256.cuh"
 #include "host.hpp"
+#include <emmintrin.h>
+#include <algorithm>
 
 namespace {
 // non-root chaining value of one leaf of leaf_size <= 1024 bytes (a single
@@ -320,23 +322,96 @@ __global__ void k_pow_sha(uint4 d0, uint4 d1, uint32_t bits, uint64_t start, uin
   if (ok) atomicMin(found, (unsigned long long)n);
 }
 
-uint64_t pow_search(const uint8_t digest[32], uint32_t bits, cudaStream_t s, unsigned long long* d_found,
-                    unsigned long long* h_found, int fn) {
+namespace {
+// One range of the search per call of `scan`, which returns the smallest valid
+// nonce in it or ~0.  The smallest valid nonce is expected near 2^bits: ranges
+// of twice that (at least 2^16, at most 2^22) in increasing order.
+template <class F>
+uint64_t pow_ranges(const uint8_t digest[32], uint32_t bits, cudaStream_t s, unsigned long long* d_found, int fn,
+                    F&& scan) {
   if (bits == 0) return 0;
   uint4 d0, d1;
   memcpy(&d0, digest, 16);
   memcpy(&d1, digest + 16, 16);
-  // the smallest valid nonce is expected near 2^bits: scan ranges of twice
-  // that (at least 2^16, at most 2^22) in increasing order
   const uint64_t chunk = 1ull << (bits + 1 < 16 ? 16 : bits + 1 > 22 ? 22 : bits + 1);
   for (uint64_t start = 0;; start += chunk) {
+    const uint64_t n = scan([&] {
+      count_launch();
+      if (fn == flock::kFnSha256)
+        k_pow_sha<<<(unsigned)(chunk / 256), 256, 0, s>>>(d0, d1, bits, start, chunk, d_found);
+      else
+        k_pow<<<(unsigned)(chunk / 256), 256, 0, s>>>(d0, d1, bits, start, chunk, d_found);
+    });
+    if (n != ~0ull) return n;
+  }
+}
+
+__global__ void k_mail(const uint32_t* __restrict__ src, int n, volatile uint64_t* words, uint32_t seq) {
+  const int t = threadIdx.x;
+  if (t < n) words[t] = (uint64_t)seq << 32 | src[t];
+}
+// a search's result, and its word ready for the next search
+__global__ void k_mail_found(unsigned long long* found, volatile uint64_t* words, uint32_t seq) {
+  const unsigned long long v = *found;
+  words[0] = (uint64_t)seq << 32 | (uint32_t)v;
+  words[1] = (uint64_t)seq << 32 | (uint32_t)(v >> 32);
+  *found = ~0ull;
+}
+
+uint32_t mail_word(const Mailbox& m, size_t i, cudaStream_t s) {
+  for (uint32_t k = 1;; k++) {
+    const uint64_t w = m.words[i];
+    if ((uint32_t)(w >> 32) == m.seq) return (uint32_t)w;
+    _mm_pause();
+    if (k % (1u << 14)) continue;
+    const cudaError_t e = cudaStreamQuery(s);
+    if (e == cudaErrorNotReady) continue;
+    CK(e);
+    if ((uint32_t)(m.words[i] >> 32) != m.seq) throw CudaError("mailbox: the stream finished without its post");
+  }
+}
+}  // namespace
+
+Mailbox mailbox_at(void* block) {
+  Mailbox m;
+  memset(block, 0, kMailBytes);  // sequence numbers start at 1
+  m.words = static_cast<uint64_t*>(block);
+  return m;
+}
+void mailbox_post(Mailbox& m, const f128* dev, size_t n, cudaStream_t s) {
+  if (n > kMailValues) throw CudaError("mailbox_post: too many values");
+  if (++m.seq == 0) m.seq = 1;
+  count_launch();
+  k_mail<<<1, (unsigned)std::max<size_t>(32, 4 * n), 0, s>>>(reinterpret_cast<const uint32_t*>(dev), (int)(4 * n),
+                                                            m.words, m.seq);
+}
+void mailbox_read(const Mailbox& m, f128* host, size_t n, cudaStream_t s) {
+  for (size_t i = 0; i < n; i++) {
+    const uint64_t w0 = mail_word(m, 4 * i, s), w1 = mail_word(m, 4 * i + 1, s);
+    const uint64_t w2 = mail_word(m, 4 * i + 2, s), w3 = mail_word(m, 4 * i + 3, s);
+    host[i] = mk(w0 | w1 << 32, w2 | w3 << 32);
+  }
+}
+
+uint64_t pow_search(const uint8_t digest[32], uint32_t bits, cudaStream_t s, unsigned long long* d_found,
+                    unsigned long long* h_found, int fn) {
+  return pow_ranges(digest, bits, s, d_found, fn, [&](auto&& launch) -> uint64_t {
     *h_found = ~0ull;
     CK(cudaMemcpyAsync(d_found, h_found, 8, cudaMemcpyHostToDevice, s));
-    count_launch();
-    if (fn == flock::kFnSha256) k_pow_sha<<<(unsigned)(chunk / 256), 256, 0, s>>>(d0, d1, bits, start, chunk, d_found);
-    else k_pow<<<(unsigned)(chunk / 256), 256, 0, s>>>(d0, d1, bits, start, chunk, d_found);
+    launch();
     CK(cudaMemcpyAsync(h_found, d_found, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (*h_found != ~0ull) return *h_found;
-  }
+    return *h_found;
+  });
+}
+uint64_t pow_search(const uint8_t digest[32], uint32_t bits, cudaStream_t s, unsigned long long* d_found, Mailbox& m,
+                    int fn) {
+  return pow_ranges(digest, bits, s, d_found, fn, [&](auto&& launch) -> uint64_t {
+    launch();
+    if (++m.seq == 0) m.seq = 1;
+    count_launch();
+    k_mail_found<<<1, 1, 0, s>>>(d_found, m.words, m.seq);
+    const uint64_t lo = mail_word(m, 0, s);
+    return lo | (uint64_t)mail_word(m, 1, s) << 32;
+  });
 }

@@ -121,7 +121,8 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   idx = dalloc<uint64_t>(1 << 16, st);
   gather = dalloc<f128>(1 << 16, st);
   d_found = dalloc<unsigned long long>(1, st);
-  h_found = static_cast<unsigned long long*>(pinned_take(8));
+  mail_block = pinned_take(kMailBytes);
+  mail = mailbox_at(mail_block);
   h_out = static_cast<f128*>(pinned_take(1024 * sizeof(f128)));
   h_stage = static_cast<uint8_t*>(pinned_take(kStageBytes));
   const Statement& S = statement(hash);
@@ -136,6 +137,7 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   CK(cudaMemcpy(bt_ptr, S.bt_ptr.data(), S.bt_ptr.size() * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(at_row, S.at_row.data(), S.at_row.size() * 2, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(bt_row, S.bt_row.data(), S.bt_row.size() * 2, cudaMemcpyHostToDevice));
+  CK(cudaMemset(d_found, 0xFF, sizeof(*d_found)));
   build_round1_tables();
   int dev_sms = 0;
   CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device));
@@ -144,7 +146,8 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   tune_ntt_plans();
   capture_commit();
   CK(cudaStreamSynchronize(st));  // the buffers exist for every stream from here on
-  device_bytes = t_alloc_bytes - bytes0;
+  // the driver's share: captured graphs, events, the stream
+  device_bytes = t_alloc_bytes - bytes0 + ((size_t)1 << 20);
 }
 
 // Tune the pass plans of every NTT shape a proof of this size runs, on this
@@ -333,7 +336,7 @@ Setup::~Setup() {
     if (L.cw) cudaFreeAsync(L.cw, st);
     if (L.tree) cudaFreeAsync(L.tree, st);
   }
-  pinned_give(h_found, 8);
+  pinned_give(mail_block, kMailBytes);
   pinned_give(h_out, 1024 * sizeof(f128));
   pinned_give(h_stage, kStageBytes);
   for (auto g : commit_graph)
@@ -377,6 +380,11 @@ void Setup::build_round1_tables() {
 void Setup::eq_table(const std::vector<f128>& r, f128* dev) { eq_build(r.data(), (int)r.size(), hone(), dev, st); }
 
 void Setup::fetch(const f128* dev, size_t n, f128* host) {
+  if (n <= kMailValues) {
+    mailbox_post(mail, dev, n, st);
+    mailbox_read(mail, host, n, st);
+    return;
+  }
   CK(cudaMemcpyAsync(host, dev, n * sizeof(f128), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
 }
@@ -388,7 +396,7 @@ uint64_t Setup::grind(Transcript& tr, uint32_t bits) {
     tr.state_digest(d);
     // a few dozen hashes on the host cost less than a round trip to the GPU
     nonce = bits <= kHostPowBits ? pow_search_host(d, bits, tr.fn())
-                                 : pow_search(d, bits, st, d_found, h_found, tr.fn());
+                                 : pow_search(d, bits, st, d_found, mail, tr.fn());
   }
   tr.nonce(nonce);
   return nonce;
@@ -438,8 +446,9 @@ void Setup::finish_openings() {
 
 H32 Setup::root_of(const uint32_t* tree, size_t n_leaves) {
   H32 r;
-  CK(cudaMemcpyAsync(r.data(), tree + 8 * (2 * n_leaves - 2), 32, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  f128 v[2];
+  fetch(reinterpret_cast<const f128*>(tree + 8 * (2 * n_leaves - 2)), 2, v);
+  memcpy(r.data(), v, 32);
   return r;
 }
 
@@ -449,7 +458,7 @@ void Setup::mark(int phase) {
 
 // -------------------------------------------------------------- prove --
 // Host buffers handed to cudaMemcpyAsync here are either pinned (h_out,
-// h_found, h_stage) and read only after a synchronisation, or pageable, which
+// h_stage) and read only after a synchronisation, or pageable, which
 // the runtime stages before the call returns: the stream needs no
 // synchronisation except where the transcript reads a device value.
 std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_dev, size_t n_blocks,
@@ -797,7 +806,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     std::vector<f128> rs;
     for (int k = 0; k <= n_log; k++) {
       // the last message is over g[0], g[1]; the final fold happens here
-      if (k == n_log) CK(cudaMemcpyAsync(h_out + 2, g, 2 * sizeof(f128), cudaMemcpyDeviceToHost, st));
+      if (k == n_log) fetch(g, 2, h_out + 2);
       fetch(so, 2, h_out);
       P.shift_rounds.push_back({h_out[0], h_out[1]});
       tr.f128v(h_out[0]);
@@ -856,9 +865,11 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     f128 last[7];
     for (int k = 0; k < n; k++) {
       // the last message is over the tables' two values; they fold here
-      if (k == n - 1)
+      if (k == n - 1) {
         for (int t = 0; t < 7; t++)
           CK(cudaMemcpyAsync(h_out + 4 + 2 * t, T.t[t], 2 * sizeof(f128), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+      }
       fetch(so, 3, h_out);
       P.mp_rounds.push_back({h_out[0], h_out[1], h_out[2]});
       for (int e = 0; e < 3; e++) tr.f128v(h_out[e]);

@@ -198,7 +198,8 @@ class Setup {
   uint8_t* tabs_r1 = nullptr;
   uint64_t* idx = nullptr;
   unsigned long long* d_found = nullptr;
-  unsigned long long* h_found = nullptr;
+  Mailbox mail;  // round messages, roots and nonces on their way to the transcript
+  void* mail_block = nullptr;
   f128* h_out = nullptr;
   uint8_t* h_stage = nullptr;
   uint32_t *at_ptr = nullptr, *bt_ptr = nullptr;
