@@ -56,18 +56,27 @@ __device__ __forceinline__ void flush(const Stage& S, int blk, int lo, int hi) {
   __syncwarp();
 }
 
+// WINDOW: only the words [lo_w, hi_w) are written
+template <bool WINDOW>
 struct RowStream {
   const Stage& S;
   uint64_t* z;  // this thread's staged rows (stride kWThreads * kStride between streams)
   uint64_t zw = 0, aw = 0, bw = 0;
-  int fill = 0;  // bits pending in the accumulators
-  int word = 8;  // next u64 index to write (bit 512 starts word 8)
+  int fill;      // bits pending in the accumulators
+  int word;      // next u64 index to write
+  int lo_w, hi_w;  // the words this thread writes
+  // from bit `pos` of the block on, writing words [ceil(pos / 64), end)
+  __device__ __forceinline__ RowStream(const Stage& S_, uint64_t* row, int pos, int end)
+      : S(S_), z(row), fill(pos & 63), word(pos >> 6), lo_w((pos + 63) >> 6), hi_w(end) {}
   __device__ __forceinline__ void emit(uint64_t zv, uint64_t av, uint64_t bv) {
     const int w = word & 15;
-    z[w] = zv;
-    z[kWThreads * kStride + w] = av;
-    z[2 * kWThreads * kStride + w] = bv;
-    if (w == 15) flush(S, word >> 4, word < 16 ? 8 : 0, 16);
+    if (!WINDOW || (word >= lo_w && word < hi_w)) {
+      z[w] = zv;
+      z[kWThreads * kStride + w] = av;
+      z[2 * kWThreads * kStride + w] = bv;
+      if (!WINDOW && w == 15) flush(S, word >> 4, word < 16 ? 8 : 0, 16);
+      if (WINDOW && (w == 15 || word + 1 == hi_w)) flush(S, word >> 4, max(lo_w - (word & ~15), 0), w + 1);
+    }
     word++;
   }
   __device__ __forceinline__ void put(int n, uint32_t zv, uint32_t av, uint32_t bv) {
@@ -96,50 +105,92 @@ struct RowStream {
 
 __device__ __forceinline__ uint32_t rr(uint32_t x, int n) { return __funnelshift_r(x, x, n); }
 
+// The block's rounds start at bit 1153 + 2000 r (512 bits of prefix, the
+// constant, 20 input words; 8 G of six 31-bit carries and two words each).
+constexpr int round_pos(int r) { return 1153 + 2000 * r; }
+
+// PARTS = 1: one thread writes its compression's whole block.  PARTS = 4: four
+// threads (of different CTAs) write a quarter of it each, and run the rounds
+// before theirs without writing rows: with few compressions there are not
+// warps enough to hide the writer's latency (2^10 compressions: 32 warps, one
+// serial writer each, 83 us), and the compression itself is a twentieth of
+// the writer's work.
+template <int PARTS>
 __device__ void compression_witness(const uint32_t cv[8], const uint32_t m_in[16], uint32_t tlo, uint32_t thi,
-                                    uint32_t blen, uint32_t flags, const Stage& S) {
+                                    uint32_t blen, uint32_t flags, const Stage& S, int part) {
   uint64_t* row = S.sm + (size_t)threadIdx.x * kStride;
-  RowStream s{S, row};
-  s.put(1, 1, 1, 1);  // constant wire at bit 512
+  // rounds [r0, r1) are this part's, and the word in which round r1 starts
+  const int r0 = PARTS == 1 ? 0 : 2 * part, r1 = PARTS == 1 || part == PARTS - 1 ? 7 : 2 * part + 2;
+  RowStream<(PARTS > 1)> s(S, row, r0 ? round_pos(r0) : 512, r1 == 7 ? 256 : (round_pos(r1) + 63) / 64);
   uint32_t m[16];
 #pragma unroll
-  for (int i = 0; i < 16; i++) { m[i] = m_in[i]; s.ident(m[i]); }
-  s.ident(tlo);
-  s.ident(thi);
-  s.ident(blen);
-  s.ident(flags);
+  for (int i = 0; i < 16; i++) m[i] = m_in[i];
+  if (r0 == 0) {
+    s.put(1, 1, 1, 1);  // constant wire at bit 512
+#pragma unroll
+    for (int i = 0; i < 16; i++) s.ident(m[i]);
+    s.ident(tlo);
+    s.ident(thi);
+    s.ident(blen);
+    s.ident(flags);
+  }
   uint32_t v[16] = {cv[0], cv[1], cv[2], cv[3], cv[4], cv[5], cv[6], cv[7],
                     b3d::kIV[0], b3d::kIV[1], b3d::kIV[2], b3d::kIV[3], tlo, thi, blen, flags};
 #define WG(A, B, C, D, X, Y)                                   \
   {                                                            \
-    uint32_t a1 = s.add(s.add(v[A], v[B]), (X));               \
+    uint32_t a1 = ADD(ADD(v[A], v[B]), (X));                   \
     uint32_t d1 = rr(v[D] ^ a1, 16);                           \
-    uint32_t c1 = s.add(v[C], d1);                             \
+    uint32_t c1 = ADD(v[C], d1);                               \
     uint32_t b1 = rr(v[B] ^ c1, 12);                           \
-    uint32_t a2 = s.add(s.add(a1, b1), (Y));                   \
+    uint32_t a2 = ADD(ADD(a1, b1), (Y));                       \
     uint32_t d2 = rr(d1 ^ a2, 8);                              \
-    uint32_t c2 = s.add(c1, d2);                               \
+    uint32_t c2 = ADD(c1, d2);                                 \
     uint32_t bn = rr(b1 ^ c2, 7);                              \
-    s.ident(bn);                                               \
-    s.ident(d2);                                               \
+    ROW(bn);                                                   \
+    ROW(d2);                                                   \
     v[A] = a2; v[B] = bn; v[C] = c2; v[D] = d2;                \
   }
-#pragma unroll 1
-  for (int r = 0; r < 7; r++) {
-    WG(0, 4, 8, 12, m[0], m[1]);
-    WG(1, 5, 9, 13, m[2], m[3]);
-    WG(2, 6, 10, 14, m[4], m[5]);
-    WG(3, 7, 11, 15, m[6], m[7]);
-    WG(0, 5, 10, 15, m[8], m[9]);
-    WG(1, 6, 11, 12, m[10], m[11]);
-    WG(2, 7, 8, 13, m[12], m[13]);
-    WG(3, 4, 9, 14, m[14], m[15]);
+#define WROUND                    \
+  WG(0, 4, 8, 12, m[0], m[1]);    \
+  WG(1, 5, 9, 13, m[2], m[3]);    \
+  WG(2, 6, 10, 14, m[4], m[5]);   \
+  WG(3, 7, 11, 15, m[6], m[7]);   \
+  WG(0, 5, 10, 15, m[8], m[9]);   \
+  WG(1, 6, 11, 12, m[10], m[11]); \
+  WG(2, 7, 8, 13, m[12], m[13]);  \
+  WG(3, 4, 9, 14, m[14], m[15]);
+  auto permute = [&] {
     uint32_t t[16] = {m[2], m[6], m[3], m[10], m[7], m[0], m[4], m[13],
                       m[1], m[11], m[12], m[5], m[9], m[14], m[15], m[8]};
 #pragma unroll
     for (int i = 0; i < 16; i++) m[i] = t[i];
+  };
+  if (PARTS > 1) {
+#define ADD(X, Y) ((X) + (Y))
+#define ROW(X)
+#pragma unroll 1
+    for (int r = 0; r < r0; r++) {
+      WROUND
+      permute();
+    }
+#undef ADD
+#undef ROW
   }
+#define ADD(X, Y) s.add((X), (Y))
+#define ROW(X) s.ident(X)
+#pragma unroll 1
+  for (int r = r0; r < r1; r++) {
+    WROUND
+    permute();
+  }
+  if (PARTS > 1 && r1 < 7) {  // the rest of the last word
+    WG(0, 4, 8, 12, m[0], m[1]);
+    return;
+  }
+#undef ADD
+#undef ROW
 #undef WG
+#undef WROUND
   uint32_t lo[8];
 #pragma unroll
   for (int w = 0; w < 8; w++) {
@@ -177,8 +228,9 @@ __device__ __forceinline__ Stage make_stage(uint64_t* sm, f128* z, f128* a, f128
 
 // CTA `cta` of the witness of 2^log2 seeded compressions (n_slots >= n_blocks
 // slots; padding slots hold the all-zero compression, blake3.rs:4631-4636)
+template <int PARTS>
 __device__ __forceinline__ void witness_seed_cta(uint64_t* sm, uint64_t seed, uint32_t log2, uint32_t n_blocks,
-                                                 uint32_t n_slots, f128* z, f128* a, f128* b, uint32_t cta) {
+                                                 uint32_t n_slots, f128* z, f128* a, f128* b, uint32_t cta, int part) {
   const Stage S = make_stage(sm, z, a, b, n_slots, cta);
   uint32_t i = cta * kWThreads + threadIdx.x;
   uint32_t cv[8], m[16], ctr = 0, blen = 0, flags = 0;
@@ -199,14 +251,15 @@ __device__ __forceinline__ void witness_seed_cta(uint64_t* sm, uint64_t seed, ui
 #pragma unroll
     for (int w = 0; w < 16; w++) m[w] = 0;
   }
-  compression_witness(cv, m, ctr, 0, blen, flags, S);
+  compression_witness<PARTS>(cv, m, ctr, 0, blen, flags, S, part);
 }
 
+template <int PARTS>
 __global__ void __launch_bounds__(kWThreads, 4) k_witness_seed(uint64_t seed, uint32_t log2, uint32_t n_blocks,
                                                            uint32_t n_slots, f128* __restrict__ z,
                                                            f128* __restrict__ a, f128* __restrict__ b) {
   extern __shared__ uint64_t wsm[];
-  witness_seed_cta(wsm, seed, log2, n_blocks, n_slots, z, a, b, blockIdx.x);
+  witness_seed_cta<PARTS>(wsm, seed, log2, n_blocks, n_slots, z, a, b, blockIdx.x, blockIdx.y);
 }
 
 // The witnesses of a batch of proofs in one launch: CTA c belongs to the job
@@ -221,14 +274,14 @@ __global__ void __launch_bounds__(kWThreads, 4) k_witness_seed_batch(const Batch
     else hi = mid - 1;
   }
   const BatchJob& J = jobs[lo];
-  witness_seed_cta(wsm, J.seed, J.log2, J.n_blocks, J.n_slots, J.z, J.a, J.b, c - (uint32_t)J.wcta0);
+  witness_seed_cta<1>(wsm, J.seed, J.log2, J.n_blocks, J.n_slots, J.z, J.a, J.b, c - (uint32_t)J.wcta0, 0);
 }
 
 // blocks: REC u32 per compression.  REC = 25: cv[8], m[16], counter_lo, with
 // counter_hi = 0, block_len = 64, flags = 11 as in the benchmark generator.
 // REC = 28: the full record cv[8], m[16], counter (u64), block_len, flags
 // (Compression, blake3.rs:1861).
-template <int REC>
+template <int REC, int PARTS>
 __global__ void __launch_bounds__(kWThreads, 4) k_witness_blocks(const uint32_t* __restrict__ blocks, uint32_t n_blocks,
                                                              uint32_t n_slots, f128* __restrict__ z,
                                                              f128* __restrict__ a, f128* __restrict__ b) {
@@ -252,22 +305,33 @@ __global__ void __launch_bounds__(kWThreads, 4) k_witness_blocks(const uint32_t*
       flags = 11;
     }
   }
-  compression_witness(cv, m, ctr, ctr_hi, blen, flags, S);
+  compression_witness<PARTS>(cv, m, ctr, ctr_hi, blen, flags, S, blockIdx.y);
 }
+
+namespace {
+// four threads per compression up to kPartSlots slots (beyond, the warps of one
+// thread each fill the SMs)
+constexpr uint32_t kPartSlots = 1u << 15;
+}  // namespace
 
 void launch_witness_seed(uint64_t seed, uint32_t log2, uint32_t n_blocks, uint32_t n_slots, f128* z, f128* a,
                          f128* b, cudaStream_t s) {
-  CK(cudaFuncSetAttribute(k_witness_seed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWitnessSmem));
+  const bool split = n_slots <= kPartSlots;
+  auto kern = split ? k_witness_seed<4> : k_witness_seed<1>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWitnessSmem));
   count_launch();
-  k_witness_seed<<<(n_slots + kWThreads - 1) / kWThreads, kWThreads, kWitnessSmem, s>>>(seed, log2, n_blocks, n_slots,
-                                                                                     z, a, b);
+  kern<<<dim3((n_slots + kWThreads - 1) / kWThreads, split ? 4 : 1), kWThreads, kWitnessSmem, s>>>(
+      seed, log2, n_blocks, n_slots, z, a, b);
 }
 void launch_witness_blocks(const uint32_t* blocks, uint32_t n_blocks, uint32_t n_slots, f128* z, f128* a, f128* b,
                            cudaStream_t s, bool records) {
-  auto kern = records ? k_witness_blocks<28> : k_witness_blocks<25>;
+  const bool split = n_slots <= kPartSlots;
+  auto kern = records ? (split ? k_witness_blocks<28, 4> : k_witness_blocks<28, 1>)
+                      : (split ? k_witness_blocks<25, 4> : k_witness_blocks<25, 1>);
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWitnessSmem));
   count_launch();
-  kern<<<(n_slots + kWThreads - 1) / kWThreads, kWThreads, kWitnessSmem, s>>>(blocks, n_blocks, n_slots, z, a, b);
+  kern<<<dim3((n_slots + kWThreads - 1) / kWThreads, split ? 4 : 1), kWThreads, kWitnessSmem, s>>>(blocks, n_blocks,
+                                                                                                   n_slots, z, a, b);
 }
 
 uint32_t witness_ctas(uint32_t n_slots) { return (n_slots + kWThreads - 1) / kWThreads; }
