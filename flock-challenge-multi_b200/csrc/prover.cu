@@ -109,7 +109,7 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   tabs_r1 = dalloc<uint8_t>(round1_tables_size(), st);
   lag = dalloc<f128>(8 * 256, st);
   const size_t kk = (size_t)1 << k_log;
-  comb = dalloc<f128>(kk, st);
+  comb = dalloc<f128>(2 * kk, st);
   zv = dalloc<f128>(kk, st);
   zv_pre = dalloc<f128>(kk, st);
   eq_inner = dalloc<f128>(kk, st);

@@ -121,27 +121,48 @@ void fold_pair_final(const f128* a_in, const f128* b_in, f128 rho, f128* out, cu
 }
 
 // ------------------------------------------------------------------ K6 --
-// comb[c] = alpha * (A^T eq)[c] + (B^T eq)[c] (+ beta at the pinned column):
-// one warp per column, its lanes striding over the column's nonzeros
-// (CSC row indices) and XOR-reducing by shuffles.
-__global__ void __launch_bounds__(256) k_lc_comb(const uint32_t* __restrict__ at_ptr,
-                                                 const uint16_t* __restrict__ at_row,
-                                                 const uint32_t* __restrict__ bt_ptr,
-                                                 const uint16_t* __restrict__ bt_row, const f128* __restrict__ eq,
-                                                 f128 alpha, f128 beta, int pin, int k, f128* __restrict__ comb) {
-  const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (c >= k) return;
-  f128 sa = mk(0, 0), sb = mk(0, 0);
-  for (uint32_t j = at_ptr[c] + lane; j < at_ptr[c + 1]; j += 32) sa = fx(sa, ldg(eq + at_row[j]));
-  for (uint32_t j = bt_ptr[c] + lane; j < bt_ptr[c + 1]; j += 32) sb = fx(sb, ldg(eq + bt_row[j]));
-  sa = warp_xor(sa);
-  sb = warp_xor(sb);
-  if (lane == 0) {
-    f128 v = fx(fmul(alpha, sa), sb);
-    if (c == pin) v = fx(v, beta);
-    st(comb + c, v);
+// comb[c] = alpha * (A^T eq)[c] + (B^T eq)[c] (+ beta at the pinned column).
+// The sums are gathers of 16-byte eq values at the columns' CSC row indices
+// (21 M of them for the BLAKE3 block).  A CTA holds one 8-byte half of the
+// table (2^14 rows; for 2^15 rows, one 4-byte quarter) in shared memory and a
+// warp sums that part of a column, its lanes striding over the nonzeros; a
+// second kernel forms the products.  Gathered from global memory, where the
+// 256 KiB table misses L1, the sums took 82 us; they take 53 us here (2^14
+// compressions; 56 and 43 us with the rows still in L2 from a proof of 2^10).
+template <class W>
+__global__ void __launch_bounds__(1024) k_lc_sums(const uint32_t* __restrict__ at_ptr,
+                                                  const uint16_t* __restrict__ at_row,
+                                                  const uint32_t* __restrict__ bt_ptr,
+                                                  const uint16_t* __restrict__ bt_row, const W* __restrict__ eq, int k,
+                                                  W* __restrict__ sums) {
+  extern __shared__ __align__(16) uint8_t lc_sm[];
+  W* T = reinterpret_cast<W*>(lc_sm);
+  constexpr int kParts = 16 / sizeof(W);
+  const int part = blockIdx.y;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) T[i] = eq[(size_t)i * kParts + part];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * blockDim.x) >> 5;
+  for (int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c < 2 * k; c += warps) {
+    const bool B = c >= k;
+    const uint32_t* ptr = (B ? bt_ptr - k : at_ptr) + c;
+    const uint16_t* row = B ? bt_row : at_row;
+    const uint32_t e = ptr[1];
+    W v = 0;
+    uint32_t j = ptr[0] + lane;
+    for (; j + 96 < e; j += 128) v ^= T[row[j]] ^ T[row[j + 32]] ^ T[row[j + 64]] ^ T[row[j + 96]];
+    for (; j < e; j += 32) v ^= T[row[j]];
+#pragma unroll
+    for (int m = 16; m; m >>= 1) v ^= __shfl_xor_sync(0xffffffffu, v, m);
+    if (lane == 0) sums[(size_t)c * kParts + part] = v;
   }
+}
+// comb: the 2 k sums in, the k values out
+__global__ void __launch_bounds__(256) k_lc_comb(f128* comb, f128 alpha, f128 beta, int pin, int k) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= k) return;
+  f128 v = fx(fmul(alpha, ld(comb + c)), ld(comb + k + c));
+  if (c == pin) v = fx(v, beta);
+  st(comb + c, v);
 }
 
 // z_vec[i] = XOR over compressions o of eq(x_outer, o) where bit i of o's
@@ -260,8 +281,26 @@ __global__ void __launch_bounds__(256) k_lc_round(f128* comb, f128* zv, int len,
 
 void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_ptr, const uint16_t* bt_row,
              const f128* eq, f128 alpha, f128 beta, int pin, int k, f128* comb, cudaStream_t s) {
-  count_launch();
-  k_lc_comb<<<k * 32 / 256, 256, 0, s>>>(at_ptr, at_row, bt_ptr, bt_row, eq, alpha, beta, pin, k, comb);
+  const int parts = k <= (1 << 14) ? 2 : 4;
+  const size_t smem = (size_t)k * 16 / parts;
+  if (smem > ((size_t)128 << 10)) throw CudaError("lc_comb: at most 2^15 rows");
+  int dev = 0, sms = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const dim3 grid(sms / parts, parts);
+  count_launch(2);
+  if (parts == 2) {
+    CK(cudaFuncSetAttribute(k_lc_sums<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 << 10));
+    k_lc_sums<uint64_t><<<grid, 1024, smem, s>>>(at_ptr, at_row, bt_ptr, bt_row,
+                                                 reinterpret_cast<const uint64_t*>(eq), k,
+                                                 reinterpret_cast<uint64_t*>(comb));
+  } else {
+    CK(cudaFuncSetAttribute(k_lc_sums<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 << 10));
+    k_lc_sums<uint32_t><<<grid, 1024, smem, s>>>(at_ptr, at_row, bt_ptr, bt_row,
+                                                 reinterpret_cast<const uint32_t*>(eq), k,
+                                                 reinterpret_cast<uint32_t*>(comb));
+  }
+  k_lc_comb<<<(k + 255) / 256, 256, 0, s>>>(comb, alpha, beta, pin, k);
 }
 void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s) {
   // compressions per CTA (a multiple of 64), sized so that the columns x

@@ -994,7 +994,7 @@ Verifier::Verifier(int device) : device_(device) {
   CK(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
   CK(cudaMalloc(&eqx_, ((size_t)1 << (kMaxKLog - kKSkip)) * sizeof(f128)));  // eq(x_inner), 2^(k_log - 6)
   CK(cudaMalloc(&eqi_, ((size_t)1 << kMaxKLog) * sizeof(f128)));  // the largest block of the statements
-  CK(cudaMalloc(&comb_, ((size_t)1 << kMaxKLog) * sizeof(f128)));
+  CK(cudaMalloc(&comb_, ((size_t)2 << kMaxKLog) * sizeof(f128)));
   CK(cudaMalloc(&kcw_, keccak_comb_scratch(3) * sizeof(f128)));
   CK(cudaMalloc(&rows_, kRowsCap));
   CK(cudaMalloc(&cvs_, kCvsCap));
