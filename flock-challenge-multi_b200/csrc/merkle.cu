@@ -62,21 +62,35 @@ __device__ __forceinline__ void parent_cv(const uint32_t* __restrict__ in, uint3
   o[1] = make_uint4(cv[4], cv[5], cv[6], cv[7]);
 }
 
-// upper levels of one tree inside one CTA (levels of at most 1024 nodes);
-// each level is read back from global memory after the barrier that
-// published it
+// upper levels of one tree inside one CTA (levels of at most 1024 nodes), each
+// level also kept in shared memory for the next
 __device__ __forceinline__ void tree_top(uint32_t* tree, size_t level_start, size_t level_len) {
-  int t = threadIdx.x;
+  __shared__ __align__(16) uint32_t cvs[512 * 8];
+  const int t = threadIdx.x;
   size_t len = level_len, start = level_start;
+  bool first = true;
   while (len > 1) {
-    size_t n = len >> 1;
-    for (size_t i = t; i < n; i += blockDim.x) {
-      uint32_t m[16], cv[8];
-      for (int k = 0; k < 16; k++) m[k] = tree[(start + 2 * i) * 8 + k];
+    const size_t n = len >> 1;
+    // 512 threads: a thread owns at most one node of a level
+    uint32_t m[16], cv[8];
+    if ((size_t)t < n) {
+      const uint4* q = reinterpret_cast<const uint4*>(first ? tree + (start + 2 * t) * 8 : cvs + 16 * t);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint4 v = q[k];
+        m[4 * k] = v.x; m[4 * k + 1] = v.y; m[4 * k + 2] = v.z; m[4 * k + 3] = v.w;
+      }
       b3d::compress(b3d::kIV, m, 0, 64, b3d::PARENT, cv);
-      for (int k = 0; k < 8; k++) tree[(start + len + i) * 8 + k] = cv[k];
+    }
+    __syncthreads();  // the level below has been read
+    if ((size_t)t < n) {
+      uint4* g = reinterpret_cast<uint4*>(tree + (start + len + t) * 8);
+      uint4* s = reinterpret_cast<uint4*>(cvs + 8 * t);
+      g[0] = s[0] = make_uint4(cv[0], cv[1], cv[2], cv[3]);
+      g[1] = s[1] = make_uint4(cv[4], cv[5], cv[6], cv[7]);
     }
     __syncthreads();
+    first = false;
     start += len;
     len = n;
   }
