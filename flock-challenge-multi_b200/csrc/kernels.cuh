@@ -78,6 +78,54 @@ __device__ __forceinline__ void block_xor_out(f128 v, f128* out) {
   __syncthreads();
 }
 
+// Small device results for a host that waits for them.  A kernel on the stream
+// writes each 32-bit word of the values to page-locked memory as one 64-bit
+// store with a sequence number beside it, and the host reads a word once its
+// number has come: no fence, no copy engine and no driver wait (a copy and a
+// stream synchronisation for the same bytes take about 4 us longer).
+constexpr size_t kMailValues = 128;
+// What a kernel that sums a round's message needs to post it itself: its last
+// CTA to finish writes n values (words == nullptr: nothing is posted).
+struct MailArgs {
+  volatile uint64_t* words = nullptr;
+  unsigned* ticket = nullptr;  // device, 0 between launches
+  uint32_t seq = 0;
+  int n = 0;
+};
+struct Mailbox {
+  volatile uint64_t* words = nullptr;  // page-locked, kMailValues * 4 of (seq << 32 | data)
+  unsigned* ticket = nullptr;          // device, 0
+  uint32_t seq = 0;
+  // the next post, of n values, by the kernel that takes the arguments
+  MailArgs next(int n) {
+    if (++seq == 0) seq = 1;
+    return {words, ticket, seq, n};
+  }
+};
+constexpr size_t kMailBytes = kMailValues * 32;
+// block: kMailBytes of page-locked memory; ticket: a zeroed device word
+Mailbox mailbox_at(void* block, unsigned* ticket);
+// n (<= kMailValues) values at dev, behind the work queued on s
+void mailbox_post(Mailbox& m, const f128* dev, size_t n, cudaStream_t s);
+// the n values of the last post (throws if the stream failed or ran dry without it)
+void mailbox_read(const Mailbox& m, f128* host, size_t n, cudaStream_t s);
+
+// The CTA that finishes last posts M.n values at src, which the CTAs of the
+// grid have accumulated into; every thread calls it after its CTA's last add.
+__device__ __forceinline__ void mail_last(const MailArgs& M, const f128* src) {
+  if (!M.words) return;
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(M.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(src);
+  for (int t = threadIdx.x; t < 4 * M.n; t += blockDim.x) M.words[t] = (uint64_t)M.seq << 32 | __ldcg(w + t);
+  if (threadIdx.x == 0) *M.ticket = 0;
+}
+
 // Merkle-path shift sumcheck (SHA-256 statement): the seven tables of a
 // y-round (ta, te, tb, gz, gxl, gxr, g_other) and the claim's eight word
 // coefficients
@@ -97,24 +145,6 @@ struct DeviceTimeouts {
 };
 const DeviceTimeouts& device_timeouts();
 void check_device_timeouts();
-
-// Small device results for a host that waits for them.  A kernel on the stream
-// writes each 32-bit word of the values to page-locked memory as one 64-bit
-// store with a sequence number beside it, and the host reads a word once its
-// number has come: no fence, no copy engine and no driver wait (a copy and a
-// stream synchronisation for the same bytes take about 4 us longer).
-constexpr size_t kMailValues = 128;
-struct Mailbox {
-  volatile uint64_t* words = nullptr;  // page-locked, kMailValues * 4 of (seq << 32 | data)
-  uint32_t seq = 0;
-};
-constexpr size_t kMailBytes = kMailValues * 32;
-// block: kMailBytes of page-locked memory
-Mailbox mailbox_at(void* block);
-// n (<= kMailValues) values at dev, behind the work queued on s
-void mailbox_post(Mailbox& m, const f128* dev, size_t n, cudaStream_t s);
-// the n values of the last post (throws if the stream failed or ran dry without it)
-void mailbox_read(const Mailbox& m, f128* host, size_t n, cudaStream_t s);
 
 // K0
 void launch_witness_seed(uint64_t seed, uint32_t log2, uint32_t n_blocks, uint32_t n_slots, f128* z, f128* a,
@@ -250,31 +280,33 @@ constexpr int kMaxEqTables = 4;
 void eq_build(const EqTable* tabs, int count, cudaStream_t s);  // one launch
 void eq_build(const f128* r, int n, f128 scale, f128* out, cudaStream_t s);
 void outer64(const f128* L, const f128* e, size_t n_e, f128* out, cudaStream_t s);
-void inner(const f128* f, const f128* g, size_t n, f128* out, int grid, cudaStream_t s);
+void inner(const f128* f, const f128* g, size_t n, f128* out, int grid, cudaStream_t s, const MailArgs& mail = {});
 size_t round1_tables_size();
 void build_round1_tables_host(const uint8_t M[64][64], const f128* phi8, void* dst);
 void zc_round1(const f128* a, const f128* b, const f128* c, const void* tabs, const f128* eqc, size_t n_blocks,
                f128* out, int grid, cudaStream_t s);
 void zc_round(int mode, const f128* a_in, const f128* b_in, f128* a_out, f128* b_out, const f128* lag, f128 rho,
               size_t n_pairs, int ns, int nm, int msh, const f128* etab, f128* out, int sms, cudaStream_t s,
-              f128* halve_out = nullptr, size_t halve_n = 0);
+              f128* halve_out = nullptr, size_t halve_n = 0, const MailArgs& mail = {});
 void fold_pair_final(const f128* a_in, const f128* b_in, f128 rho, f128* out, cudaStream_t s);
 // k: columns of the block matrices (2^k_log); comb: room for 2 k values
 void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_ptr, const uint16_t* bt_row,
              const f128* eq, f128 alpha, f128 beta, int pin, int k, f128* comb, cudaStream_t s);
 void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s);
-void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s);
+void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s,
+              const MailArgs& mail = {});
 // s_hat_v of the ab claim from the block-folded z (2^k_log values)
 void ring_shat_ab(const f128* zv_pre, const f128* eqt, int k_log, f128* out, cudaStream_t s);
 // f, msg (optional): also XOR the first Ligerito message over (f, b_combined)
 // into msg[0..2) (zeroed), the values k_lig_msg gives for the same pairs
 void ring_bcombined_ct(const f128* elo0, const f128* ehi0, const f128* elo1, const f128* ehi1, const f128* L0,
                        const f128* L1, int lo_bits, size_t n_chunks, f128* out, int sms, cudaStream_t s,
-                       const f128* f = nullptr, f128* msg = nullptr);
+                       const f128* f = nullptr, f128* msg = nullptr, const MailArgs& mail = {});
 // sms: the SMs a launch may fill (one wave of resident CTAs on them)
-void lig_msg(const f128* f, const f128* b, size_t n_pairs, f128* out, int sms, cudaStream_t s);
+void lig_msg(const f128* f, const f128* b, size_t n_pairs, f128* out, int sms, cudaStream_t s,
+             const MailArgs& mail = {});
 void lig_fold_msg(const f128* f, const f128* b, f128* fo, f128* bo, f128 r, size_t n_pairs_out, bool emit, f128* out,
-                  int sms, cudaStream_t s);
+                  int sms, cudaStream_t s, const MailArgs& mail = {});
 // hash chain: region fold of every instance's cv / out_lo words (g = [In | Out],
 // 2 n_inst values) and the packed-direct claim's scatter into b_combined;
 // per: packed words per block (2^(k_log - 7))

@@ -386,18 +386,19 @@ uint32_t mail_word(const Mailbox& m, size_t i, cudaStream_t s) {
 }
 }  // namespace
 
-Mailbox mailbox_at(void* block) {
+Mailbox mailbox_at(void* block, unsigned* ticket) {
   Mailbox m;
   memset(block, 0, kMailBytes);  // sequence numbers start at 1
   m.words = static_cast<uint64_t*>(block);
+  m.ticket = ticket;
   return m;
 }
 void mailbox_post(Mailbox& m, const f128* dev, size_t n, cudaStream_t s) {
   if (n > kMailValues) throw CudaError("mailbox_post: too many values");
-  if (++m.seq == 0) m.seq = 1;
+  const MailArgs a = m.next((int)n);
   count_launch();
   k_mail<<<1, (unsigned)std::max<size_t>(32, 4 * n), 0, s>>>(reinterpret_cast<const uint32_t*>(dev), (int)(4 * n),
-                                                            m.words, m.seq);
+                                                            a.words, a.seq);
 }
 void mailbox_read(const Mailbox& m, f128* host, size_t n, cudaStream_t s) {
   for (size_t i = 0; i < n; i++) {
@@ -422,9 +423,9 @@ uint64_t pow_search(const uint8_t digest[32], uint32_t bits, cudaStream_t s, uns
                     int fn) {
   return pow_ranges(digest, bits, s, d_found, fn, [&](auto&& launch) -> uint64_t {
     launch();
-    if (++m.seq == 0) m.seq = 1;
+    const MailArgs a = m.next(1);
     count_launch();
-    k_mail_found<<<1, 1, 0, s>>>(d_found, m.words, m.seq);
+    k_mail_found<<<1, 1, 0, s>>>(d_found, a.words, a.seq);
     const uint64_t lo = mail_word(m, 0, s);
     return lo | (uint64_t)mail_word(m, 1, s) << 32;
   });

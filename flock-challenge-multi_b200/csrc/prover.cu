@@ -122,7 +122,8 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   gather = dalloc<f128>(1 << 16, st);
   d_found = dalloc<unsigned long long>(1, st);
   mail_block = pinned_take(kMailBytes);
-  mail = mailbox_at(mail_block);
+  d_ticket = dalloc<unsigned>(1, st);
+  mail = mailbox_at(mail_block, d_ticket);
   h_out = static_cast<f128*>(pinned_take(1024 * sizeof(f128)));
   h_stage = static_cast<uint8_t*>(pinned_take(kStageBytes));
   const Statement& S = statement(hash);
@@ -138,6 +139,7 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   CK(cudaMemcpy(at_row, S.at_row.data(), S.at_row.size() * 2, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(bt_row, S.bt_row.data(), S.bt_row.size() * 2, cudaMemcpyHostToDevice));
   CK(cudaMemset(d_found, 0xFF, sizeof(*d_found)));
+  CK(cudaMemset(d_ticket, 0, sizeof(*d_ticket)));
   build_round1_tables();
   int dev_sms = 0;
   CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device));
@@ -328,7 +330,7 @@ void batch_commit(const std::vector<Setup*>& setups, const std::vector<uint64_t>
 Setup::~Setup() {
   cudaStreamSynchronize(st);
   void* ptrs[] = {z, a, b, cw0, tree0, pp[0], pp[1], pp[2], pp[3], eqbuf[0], zv_pre, induce_buf, out, blocks_buf, records_buf,
-                  tabs_r1, lag, comb, zv, eq_inner, bc_tabs, idx, gather, d_found, at_ptr, bt_ptr,
+                  tabs_r1, lag, comb, zv, eq_inner, bc_tabs, idx, gather, d_found, d_ticket, at_ptr, bt_ptr,
                   at_row, bt_row, kc_w};
   for (void* p : ptrs)
     if (p) cudaFreeAsync(p, st);
@@ -637,13 +639,13 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
       nxt_len = etab_len / 2;
     }
     f128* o = next_out(1);
-    zc_round(mode, ain, bin, aout, bout, lag, rho, n_pairs, ns, nm, med0 - 9, etab, o, gs, st, nxt, nxt_len);
+    zc_round(mode, ain, bin, aout, bout, lag, rho, n_pairs, ns, nm, med0 - 9, etab, o, gs, st, nxt, nxt_len, mail.next(8));
     if (nxt) {
       etab = nxt;
       etab_len = nxt_len;
       etab_off += nxt_len;
     }
-    fetch(o, 8, h_out);
+    mailbox_read(mail, h_out, 8, st);
     f128 g1 = mk(0, 0), gi = mk(0, 0);
     for (int js = 0; js < (1 << ns); js++) {
       g1 = fx(g1, hmul(K[js], h_out[2 * js]));
@@ -752,17 +754,18 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   int len = kk;
   // the round kernel adds its message atomically into a fresh slot
   f128* lo_ = next_out(1);
-  lc_round(comb, zv, len, false, mk(0, 0), true, lo_, st);
+  lc_round(comb, zv, len, false, mk(0, 0), true, lo_, st, mail.next(2));
   for (int k = 0; k < ir; k++) {
-    fetch(lo_, 2, h_out);
+    mailbox_read(mail, h_out, 2, st);
     P.lc_rounds.push_back({h_out[0], h_out[1]});
     tr.f128v(h_out[0]);
     tr.f128v(h_out[1]);
     f128 rk = tr.sample();
     rr.push_back(rk);
     len >>= 1;
-    if (k + 1 < ir) lo_ = next_out(1);
-    lc_round(comb, zv, len, true, rk, k + 1 < ir, lo_, st);
+    const bool more = k + 1 < ir;
+    if (more) lo_ = next_out(1);
+    lc_round(comb, zv, len, true, rk, more, lo_, st, more ? mail.next(2) : MailArgs{});
   }
   P.z_partial.resize(64);
   fetch(zv, 64, P.z_partial.data());
@@ -802,12 +805,12 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     CK(cudaMemcpyAsync(w, &alpha, sizeof(f128), cudaMemcpyHostToDevice, st));
     int len = (int)(2 * N);
     f128* so = next_out(1);
-    lc_round(w, g, len, false, mk(0, 0), true, so, st);
+    lc_round(w, g, len, false, mk(0, 0), true, so, st, mail.next(2));
     std::vector<f128> rs;
     for (int k = 0; k <= n_log; k++) {
       // the last message is over g[0], g[1]; the final fold happens here
+      mailbox_read(mail, h_out, 2, st);
       if (k == n_log) fetch(g, 2, h_out + 2);
-      fetch(so, 2, h_out);
       P.shift_rounds.push_back({h_out[0], h_out[1]});
       tr.f128v(h_out[0]);
       tr.f128v(h_out[1]);
@@ -816,7 +819,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
       if (k < n_log) {
         len >>= 1;
         so = next_out(1);
-        lc_round(w, g, len, true, rk, true, so, st);
+        lc_round(w, g, len, true, rk, true, so, st, mail.next(2));
       } else {
         pd_value = fx(h_out[2], hmul(rk, fx(h_out[3], h_out[2])));
       }
@@ -987,7 +990,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     // Ligerito message (over z and b_combined) is summed in the same pass
     if (!chain && !merkle && lo_bits >= 1) first_msg = next_out(1);
     ring_bcombined_ct(d, d + nlo, d + nlo + nhi, d + 2 * nlo + nhi, bc_tabs, bc_tabs + 4096, lo_bits, nhi, pp[1],
-                      gs, st, first_msg ? z : nullptr, first_msg);
+                      gs, st, first_msg ? z : nullptr, first_msg, first_msg ? mail.next(2) : MailArgs{});
   }
   if (chain) {
     // b_combined += gpd eq(point): words w < 2R of block i (R packed words
@@ -1029,7 +1032,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   size_t flen = n_words;
   f128* mo = nullptr;  // the slot of the pending message
   auto push_msg = [&]() {
-    fetch(mo, 2, h_out);
+    mailbox_read(mail, h_out, 2, st);
     P.sc_msgs.push_back({h_out[0], h_out[1]});
     tr.f128v(h_out[0]);
     tr.f128v(h_out[1]);
@@ -1038,14 +1041,14 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     mo = first_msg;  // summed with b_combined (no next_out since: the slot is intact)
   } else {
     mo = next_out(1);
-    lig_msg(f, bb, flen / 2, mo, gs, st);
+    lig_msg(f, bb, flen / 2, mo, gs, st, mail.next(2));
   }
   push_msg();
   auto fold_round = [&](int bits) -> f128 {
     if (bits > 0) P.fold_nonces.push_back(grind(tr, (uint32_t)bits));
     f128 rch = tr.sample();
     mo = next_out(1);
-    lig_fold_msg(f, bb, fo, bo, rch, flen / 4, true, mo, gs, st);
+    lig_fold_msg(f, bb, fo, bo, rch, flen / 4, true, mo, gs, st, mail.next(2));
     // after the first fold f lives in the ping-pong pair (pp[0], pp[2]) / (pp[1], pp[3])
     if (f == z) { f = fo; fo = pp[0]; }
     else std::swap(f, fo);
@@ -1056,7 +1059,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   };
   auto introduce = [&](const f128* bnew) {
     mo = next_out(1);
-    lig_msg(f, bnew, flen / 2, mo, gs, st);
+    lig_msg(f, bnew, flen / 2, mo, gs, st, mail.next(2));
     push_msg();
     f128 be = tr.sample();
     axpy(bb, bnew, be, flen, st);
@@ -1068,9 +1071,9 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
       f128* eqz = scratch_eq();
       eq_table(zp, eqz);
       f128* io = next_out(1);
-      inner(f, eqz, flen, io, G, st);
+      inner(f, eqz, flen, io, G, st, mail.next(1));
       f128 y;
-      fetch(io, 1, &y);
+      mailbox_read(mail, &y, 1, st);
       P.ood.push_back(y);
       tr.f128v(y);
       introduce(eqz);

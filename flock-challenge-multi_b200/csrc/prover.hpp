@@ -200,6 +200,7 @@ class Setup {
   unsigned long long* d_found = nullptr;
   Mailbox mail;  // round messages, roots and nonces on their way to the transcript
   void* mail_block = nullptr;
+  unsigned* d_ticket = nullptr;
   f128* h_out = nullptr;
   uint8_t* h_stage = nullptr;
   uint32_t *at_ptr = nullptr, *bt_ptr = nullptr;

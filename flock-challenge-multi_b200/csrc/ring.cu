@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256, 3) k_bcombined_msg(const f128* __restrict
                                                           const f128* __restrict__ elo1, const f128* __restrict__ ehi1,
                                                           const f128* __restrict__ L0, const f128* __restrict__ L1,
                                                           int lo_bits, size_t n_chunks, const f128* __restrict__ f,
-                                                          f128* __restrict__ out, f128* __restrict__ msg) {
+                                                          f128* __restrict__ out, f128* __restrict__ msg, MailArgs mail) {
   extern __shared__ __align__(16) uint8_t sm[];
   Tab4* C = reinterpret_cast<Tab4*>(sm);
   __shared__ f128 img[256];
@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(256, 3) k_bcombined_msg(const f128* __restrict
   }
   block_xor_out(reduce(u0), msg);
   block_xor_out(reduce(u2), msg + 1);
+  mail_last(mail, msg);
 }
 
 void ring_shat_ab(const f128* zv_pre, const f128* eqt, int k_log, f128* out, cudaStream_t s) {
@@ -121,7 +122,7 @@ void ring_shat_ab(const f128* zv_pre, const f128* eqt, int k_log, f128* out, cud
 
 void ring_bcombined_ct(const f128* elo0, const f128* ehi0, const f128* elo1, const f128* ehi1, const f128* L0,
                        const f128* L1, int lo_bits, size_t n_chunks, f128* out, int sms, cudaStream_t s,
-                       const f128* f, f128* msg) {
+                       const f128* f, f128* msg, const MailArgs& mail) {
   size_t smem = 2 * kTab4Bytes;
   if (f && msg) {
     if (lo_bits < 1) throw CudaError("ring_bcombined_ct: the message needs chunks of at least 2 values");
@@ -129,7 +130,7 @@ void ring_bcombined_ct(const f128* elo0, const f128* ehi0, const f128* elo1, con
     const size_t grid = (size_t)resident_grid((const void*)k_bcombined_msg, 256, smem, sms);
     count_launch();
     k_bcombined_msg<<<(unsigned)std::min<size_t>(n_chunks, grid), 256, smem, s>>>(elo0, ehi0, elo1, ehi1, L0, L1,
-                                                                                 lo_bits, n_chunks, f, out, msg);
+                                                                                 lo_bits, n_chunks, f, out, msg, mail);
     return;
   }
   CK(cudaFuncSetAttribute(k_bcombined_ct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -99,11 +99,12 @@ __global__ void k_axpy(f128* __restrict__ out, const f128* __restrict__ x, f128 
 }
 
 // out[0] ^= sum_i f[i] g[i]
-__global__ void k_inner(const f128* __restrict__ f, const f128* __restrict__ g, size_t n, f128* out) {
+__global__ void k_inner(const f128* __restrict__ f, const f128* __restrict__ g, size_t n, f128* out, MailArgs mail) {
   u256 acc = zero256();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     acc_wide(acc, mul_wide(ld(f + i), ld(g + i)));
   block_xor_out(reduce(acc), out);
+  mail_last(mail, out);
 }
 
 // ------------------------------------------------------------------ K5 --
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(256) k_lc_zvec(const uint16_t* __restrict__ z,
 // them, so the grid needs no synchronisation; the message is XOR-reduced per
 // CTA and added atomically (out must be zero).
 __global__ void __launch_bounds__(256) k_lc_round(f128* comb, f128* zv, int len, int do_fold, f128 r, int emit,
-                                                  f128* out) {
+                                                  f128* out, MailArgs mail) {
   const int h = len >> 1;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   f128 q1 = mk(0, 0), qi = mk(0, 0);
@@ -277,6 +278,7 @@ __global__ void __launch_bounds__(256) k_lc_round(f128* comb, f128* zv, int len,
   if (!emit) return;
   block_xor_out(q1, out);
   block_xor_out(qi, out + 1);
+  mail_last(mail, out);
 }
 
 void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_ptr, const uint16_t* bt_row,
@@ -313,16 +315,17 @@ void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv
   count_launch();
   k_lc_zvec<<<grid, 256, 0, s>>>((const uint16_t*)z, eqo, n_outer, (int)chunk, 1 << (k_log - 4), zv);
 }
-void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s) {
+void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s,
+              const MailArgs& mail) {
   const int threads = std::max(1, len / 2);
   count_launch();
-  k_lc_round<<<(threads + 255) / 256, 256, 0, s>>>(comb, zv, len, fold, r, emit, out);
+  k_lc_round<<<(threads + 255) / 256, 256, 0, s>>>(comb, zv, len, fold, r, emit, out, mail);
 }
 
 // ------------------------------------------------------------------ K7 --
 // ------------------------------------------------------------------ K8 --
 __global__ void __launch_bounds__(256) k_lig_msg(const f128* __restrict__ f, const f128* __restrict__ b,
-                                                 size_t n_pairs, f128* __restrict__ out) {
+                                                 size_t n_pairs, f128* __restrict__ out, MailArgs mail) {
   u256 u0 = zero256(), u2 = zero256();
   for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_pairs; j += (size_t)gridDim.x * blockDim.x) {
     f128 f0 = ld(f + 2 * j), f1 = ld(f + 2 * j + 1), b0 = ld(b + 2 * j), b1 = ld(b + 2 * j + 1);
@@ -331,6 +334,7 @@ __global__ void __launch_bounds__(256) k_lig_msg(const f128* __restrict__ f, con
   }
   block_xor_out(reduce(u0), out);
   block_xor_out(reduce(u2), out + 1);
+  mail_last(mail, out);
 }
 
 // fold f and b at r (LSB binding), then emit the next message on the folded
@@ -338,7 +342,8 @@ __global__ void __launch_bounds__(256) k_lig_msg(const f128* __restrict__ f, con
 template <bool TAB>
 __global__ void __launch_bounds__(256) k_lig_fold_msg(const f128* __restrict__ f, const f128* __restrict__ b,
                                                       f128* __restrict__ fo, f128* __restrict__ bo, f128 r,
-                                                      size_t n_pairs_out, int emit, f128* __restrict__ out) {
+                                                      size_t n_pairs_out, int emit, f128* __restrict__ out,
+                                                      MailArgs mail) {
   extern __shared__ __align__(16) uint8_t sm[];
   MulTab8* rt = reinterpret_cast<MulTab8*>(sm);
   if (TAB) multab_build(rt, r);
@@ -360,6 +365,7 @@ __global__ void __launch_bounds__(256) k_lig_fold_msg(const f128* __restrict__ f
   if (emit) {
     block_xor_out(reduce(u0), out);
     block_xor_out(reduce(u2), out + 1);
+    mail_last(mail, out);
   }
 }
 
@@ -411,21 +417,21 @@ void sc3_round(const f128* a, const f128* b, const f128* e, f128* ao, f128* bo, 
 }
 
 // sms: the SMs the launch may fill (one wave of resident CTAs on them)
-void lig_msg(const f128* f, const f128* b, size_t n_pairs, f128* out, int sms, cudaStream_t s) {
+void lig_msg(const f128* f, const f128* b, size_t n_pairs, f128* out, int sms, cudaStream_t s, const MailArgs& mail) {
   const int grid = resident_grid((const void*)k_lig_msg, 256, 0, sms);
-  count_launch(); k_lig_msg<<<grid, 256, 0, s>>>(f, b, n_pairs, out);
+  count_launch(); k_lig_msg<<<grid, 256, 0, s>>>(f, b, n_pairs, out, mail);
 }
 void lig_fold_msg(const f128* f, const f128* b, f128* fo, f128* bo, f128 r, size_t n_pairs_out, bool emit, f128* out,
-                  int sms, cudaStream_t s) {
+                  int sms, cudaStream_t s, const MailArgs& mail) {
   count_launch();
   if (n_pairs_out >= (1u << 14)) {
     size_t smem = sizeof(MulTab8);
     CK(cudaFuncSetAttribute(k_lig_fold_msg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int grid = resident_grid((const void*)k_lig_fold_msg<true>, 256, smem, sms);
-    k_lig_fold_msg<true><<<grid, 256, smem, s>>>(f, b, fo, bo, r, n_pairs_out, emit, out);
+    k_lig_fold_msg<true><<<grid, 256, smem, s>>>(f, b, fo, bo, r, n_pairs_out, emit, out, mail);
   } else {
     const int grid = resident_grid((const void*)k_lig_fold_msg<false>, 256, 0, sms);
-    k_lig_fold_msg<false><<<grid, 256, 0, s>>>(f, b, fo, bo, r, n_pairs_out, emit, out);
+    k_lig_fold_msg<false><<<grid, 256, 0, s>>>(f, b, fo, bo, r, n_pairs_out, emit, out, mail);
   }
 }
 void eq_build(const EqTable* tabs, int count, cudaStream_t s) {
@@ -460,6 +466,6 @@ void outer64(const f128* L, const f128* e, size_t n_e, f128* out, cudaStream_t s
 void axpy(f128* out, const f128* x, f128 beta, size_t n, cudaStream_t s) {
   count_launch(); k_axpy<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, x, beta, n);
 }
-void inner(const f128* f, const f128* g, size_t n, f128* out, int grid, cudaStream_t s) {
-  count_launch(); k_inner<<<grid, 256, 0, s>>>(f, g, n, out);
+void inner(const f128* f, const f128* g, size_t n, f128* out, int grid, cudaStream_t s, const MailArgs& mail) {
+  count_launch(); k_inner<<<grid, 256, 0, s>>>(f, g, n, out, mail);
 }

@@ -50,6 +50,7 @@ struct ZcArgs {
   f128* out;
   f128* halve_out;   // next round's table: etab with its lowest variable summed out
   size_t halve_n;    // (0: none)
+  MailArgs mail;
 };
 
 __device__ __forceinline__ f128 lag_lookup(const f128* lag, uint64_t row) {
@@ -179,6 +180,7 @@ __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
     for (int k = 0; k < (int)(blockDim.x >> 5); k++) x = fx(x, red[k][threadIdx.x]);
     atomic_xor128(A.out + threadIdx.x, x);
   }
+  mail_last(A.mail, A.out);
 }
 }  // namespace
 
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
 // launch may fill (one wave of resident CTAs on them).
 void zc_round(int mode, const f128* a_in, const f128* b_in, f128* a_out, f128* b_out, const f128* lag, f128 rho,
               size_t n_pairs, int ns, int nm, int msh, const f128* etab, f128* out, int sms, cudaStream_t s,
-              f128* halve_out, size_t halve_n) {
+              f128* halve_out, size_t halve_n, const MailArgs& mail) {
   if (ns < 0 || ns > 2 || nm < 0 || nm > 4 || msh < 0 || (nm > 0 && (((1 << nm) - 1) << msh) >= 64))
     throw CudaError("zc_round: bad eq structure");
   if (n_pairs > ((size_t)1 << 30)) throw CudaError("zc_round: too many pairs");
@@ -198,6 +200,7 @@ void zc_round(int mode, const f128* a_in, const f128* b_in, f128* a_out, f128* b
   A.n_pairs = (uint32_t)n_pairs; A.ns = ns; A.nm = nm; A.msh = msh;
   A.etab = etab; A.out = out;
   A.halve_out = halve_out; A.halve_n = halve_n;
+  A.mail = mail;
   // the window table pays from about 2^14 folded pairs on (k_lig_fold_msg's line too)
   const bool plain = mode == 2 && n_pairs < ((size_t)1 << 14);
   const size_t smem = mode == 0 ? 2048 * sizeof(f128) : mode == 1 ? 4096 * sizeof(f128) : plain ? 0 : sizeof(MulTab8);
