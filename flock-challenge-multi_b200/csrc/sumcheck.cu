@@ -166,85 +166,6 @@ __global__ void __launch_bounds__(256) k_lc_comb(f128* comb, f128 alpha, f128 be
   st(comb + c, v);
 }
 
-// z_vec[i] = XOR over compressions o of eq(x_outer, o) where bit i of o's
-// 2^k_log-bit block is set (lincheck.rs:2423 partial_fold_packed_z_block_major).
-// A CTA owns 4096 bit positions (a quarter of a 2^14-bit block, an eighth of
-// a 2^15-bit one) and a run of compressions; a thread owns 16 positions (one
-// u16 of each block).  For
-// every 8 compressions the CTA builds the 256 subset sums of their eq
-// weights; a thread transposes its 8 u16 words into 16 bytes (bit k of byte
-// p = bit p of compression k) and XORs in one table entry per position.
-namespace {
-constexpr int kZvGroups = 8;  // 8-compression tables built per barrier pair
-
-__device__ __forceinline__ uint64_t transpose8x8(uint64_t x) {
-  uint64_t t;
-  t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
-  x = x ^ t ^ (t << 7);
-  t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
-  x = x ^ t ^ (t << 14);
-  t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
-  x = x ^ t ^ (t << 28);
-  return x;
-}
-}  // namespace
-
-__global__ void __launch_bounds__(256) k_lc_zvec(const uint16_t* __restrict__ z, const f128* __restrict__ eqo,
-                                                 size_t n_outer, int chunk, int bw, f128* __restrict__ zv) {
-  __shared__ __align__(16) f128 T[kZvGroups][256];
-  const int col = blockIdx.x;  // 4096-bit column of the block (bw u16 per block)
-  const int t = threadIdx.x;
-  const size_t o0 = (size_t)blockIdx.y * chunk;
-  const size_t o1 = o0 + chunk < n_outer ? o0 + chunk : n_outer;
-  f128 acc[16];
-#pragma unroll
-  for (int p = 0; p < 16; p++) acc[p] = mk(0, 0);
-  for (size_t ob = o0; ob < o1; ob += 8 * kZvGroups) {
-    __syncthreads();
-    // entry v of table g: XOR of eq(o) over the set bits k of v, o = ob + 8g + k
-#pragma unroll 1
-    for (int g = 0; g < kZvGroups; g++) {
-      f128 v = mk(0, 0);
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const size_t o = ob + 8 * g + k;
-        if (((t >> k) & 1) && o < o1) v = fx(v, ldg(eqo + o));
-      }
-      st(&T[g][t], v);
-    }
-    __syncthreads();
-    // the next group's words are loaded while the current one is folded in
-    uint32_t r[8], rn[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) r[k] = ob + k < o1 ? z[(ob + k) * bw + col * 256 + t] : 0u;
-#pragma unroll 1
-    for (int g = 0; g < kZvGroups; g++) {
-      const size_t og = ob + 8 * g;
-      if (og >= o1) break;
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const size_t o = og + 8 + k;
-        rn[k] = (g + 1 < kZvGroups && o < o1) ? z[o * bw + col * 256 + t] : 0u;
-      }
-      const uint32_t t01 = __byte_perm(r[0], r[1], 0x5140), t23 = __byte_perm(r[2], r[3], 0x5140);
-      const uint32_t t45 = __byte_perm(r[4], r[5], 0x5140), t67 = __byte_perm(r[6], r[7], 0x5140);
-      const uint64_t lo = transpose8x8((uint64_t)__byte_perm(t01, t23, 0x5410) |
-                                       ((uint64_t)__byte_perm(t45, t67, 0x5410) << 32));
-      const uint64_t hi = transpose8x8((uint64_t)__byte_perm(t01, t23, 0x7632) |
-                                       ((uint64_t)__byte_perm(t45, t67, 0x7632) << 32));
-#pragma unroll
-      for (int p = 0; p < 8; p++) {
-        acc[p] = fx(acc[p], ld(&T[g][(lo >> (8 * p)) & 0xFF]));
-        acc[8 + p] = fx(acc[8 + p], ld(&T[g][(hi >> (8 * p)) & 0xFF]));
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) r[k] = rn[k];
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < 16; p++) atomic_xor128(zv + col * 4096 + 16 * t + p, acc[p]);
-}
-
 // One lincheck round (top binding): with do_fold, fold comb and zv (2 len
 // values each) at r into their first len values; with emit, add the
 // message over the (folded) pairs (i, i + len/2) into out[0..2):
@@ -303,17 +224,6 @@ void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_
                                                  reinterpret_cast<uint32_t*>(comb));
   }
   k_lc_comb<<<(k + 255) / 256, 256, 0, s>>>(comb, alpha, beta, pin, k);
-}
-void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s) {
-  // compressions per CTA (a multiple of 64), sized so that the columns x
-  // chunks fill one wave of resident CTAs
-  const size_t cols = (size_t)1 << (k_log - 12);
-  const size_t slots = (size_t)resident_grid((const void*)k_lc_zvec, 256, 0, sms);
-  const size_t rows = std::max<size_t>(1, slots / cols);
-  const size_t chunk = std::max<size_t>(64, ((n_outer + rows - 1) / rows + 63) / 64 * 64);
-  dim3 grid((unsigned)cols, (unsigned)((n_outer + chunk - 1) / chunk));
-  count_launch();
-  k_lc_zvec<<<grid, 256, 0, s>>>((const uint16_t*)z, eqo, n_outer, (int)chunk, 1 << (k_log - 4), zv);
 }
 void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s,
               const MailArgs& mail) {
