@@ -767,6 +767,13 @@ std::vector<std::vector<std::pair<int, int>>> candidate_splits_t(int lanes, int 
   return out;
 }
 
+// From 2^kTensorMinLog positions on there are tiles enough for the SMs and the
+// tensor-core passes are the fastest of all kinds (2^12 positions x 64 lanes:
+// 0.049 ms against 0.057 ms for the best mix of the others; 2^14: 0.121 / 0.167;
+// 2^20: 7.44 / 11.8 ms; 2^10: 0.028 against 0.026 ms for the integer products),
+// so only their splits are timed there.
+constexpr int kTensorMinLog = 12;
+
 // the warp-per-pair shapes of a pass of R layers: (threads, kind) with the
 // tile and every warp's table within one CTA's shared memory
 std::vector<NttPass> candidate_shapes_w(int lanes, int l0, int R) {
@@ -831,11 +838,8 @@ NttPlan default_plan(int log_d, int lanes, int layer_begin) {
   NttPlan plan;
   const int n_layers = log_d - layer_begin;
   if (n_layers <= 0) return plan;
-  // 64 lanes: the tensor-core passes, once there are tiles enough for the SMs
-  // (2^12 positions: 0.049 ms against 0.064 ms for the integer products; 2^10:
-  // 0.028 against 0.026 ms)
   const auto tensor = candidate_splits_t(lanes, layer_begin, n_layers);
-  if (!tensor.empty() && log_d >= 12) {
+  if (!tensor.empty() && log_d >= kTensorMinLog) {
     for (auto& pr : tensor[0]) plan.push_back({pr.first, pr.second, 6, 128, 3});
     return plan;
   }
@@ -991,10 +995,15 @@ NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaS
   std::map<std::pair<int, int>, std::pair<NttPass, double>> best_pass;  // (l0, R) -> fastest shape
   NttPlan best_plan;
   double best_total = 1e300;
-  auto splits = candidate_splits(layer_begin, n_layers);
-  for (auto& sp : candidate_splits_w(layer_begin, n_layers))
-    if (std::find(splits.begin(), splits.end(), sp) == splits.end()) splits.push_back(sp);
-  for (auto& sp : candidate_splits_t(lanes, layer_begin, n_layers))
+  const auto tensor = candidate_splits_t(lanes, layer_begin, n_layers);
+  const bool tensor_only = !tensor.empty() && log_d >= kTensorMinLog;
+  std::vector<std::vector<std::pair<int, int>>> splits;
+  if (!tensor_only) {
+    splits = candidate_splits(layer_begin, n_layers);
+    for (auto& sp : candidate_splits_w(layer_begin, n_layers))
+      if (std::find(splits.begin(), splits.end(), sp) == splits.end()) splits.push_back(sp);
+  }
+  for (auto& sp : tensor)
     if (std::find(splits.begin(), splits.end(), sp) == splits.end()) splits.push_back(sp);
   for (auto& split : splits) {
     NttPlan plan;
@@ -1005,9 +1014,12 @@ NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaS
         NttPass bp{};
         double bt = 1e300;
         std::vector<NttPass> shapes;
-        if (pr.second <= kMaxR + 1)
-          for (auto& sh : candidate_shapes(lanes, pr.second)) shapes.push_back({pr.first, pr.second, sh.first, sh.second});
-        for (auto& ps : candidate_shapes_w(lanes, pr.first, pr.second)) shapes.push_back(ps);
+        if (!tensor_only) {
+          if (pr.second <= kMaxR + 1)
+            for (auto& sh : candidate_shapes(lanes, pr.second))
+              shapes.push_back({pr.first, pr.second, sh.first, sh.second});
+          for (auto& ps : candidate_shapes_w(lanes, pr.first, pr.second)) shapes.push_back(ps);
+        }
         if (lanes % 64 == 0 && pr.second >= 2 && pr.second <= kMaxRt && tensor_safe(log_d))
           shapes.push_back({pr.first, pr.second, 6, 128, 3});
         for (auto& ps : shapes) {
