@@ -126,6 +126,46 @@ __device__ __forceinline__ void mail_last(const MailArgs& M, const f128* src) {
   if (threadIdx.x == 0) *M.ticket = 0;
 }
 
+// ---- short rounds: four lanes a pair ----
+// (at most this many pairs: the lanes of 2^14 pairs are a wave of 256 CTAs)
+constexpr int kQuadPairs = 1 << 14;
+// A round over few pairs is a chain of field products (the folds, the message,
+// a weight) of a microsecond and more each.  One thread a pair runs four folds
+// and two message products one behind the other; with lane q of four folding
+// one of the pair's values (x0, x1, y0, y1) and two of them one message
+// product each, the chain is one product a step.  A Ligerito fold round takes
+// 6.5 us where one thread a pair took 9.4, a lincheck round 5.8 (9.4), a
+// zerocheck round 9 (14.5).
+// The message factors of a lane that holds v (its value of the pair): lanes q
+// and q ^ 2 return the same product, of x1 y1 for odd q and (x0 + x1)(y0 + y1)
+// for even q, or of x0 y0 and the sums with the roles swapped (LOW).
+template <bool LOW>
+__device__ __forceinline__ void quad_factors(f128 v, int q, f128& x, f128& y) {
+  const f128 s = mk(v.lo ^ shfl_xor64(v.lo, 1), v.hi ^ shfl_xor64(v.hi, 1));
+  x = (q & 1) != LOW ? v : s;
+  y = mk(shfl_xor64(x.lo, 2), shfl_xor64(x.hi, 2));
+}
+// XOR of v over the CTA's threads of lane class (threadIdx mod N) into out[class]
+// for the classes that `to` maps to 0.. (N <= 32, a power of two; every thread
+// calls it).
+template <int N, class F>
+__device__ __forceinline__ void block_xor_classes(f128 v, f128* out, F to) {
+  __shared__ f128 red[8][N];
+#pragma unroll
+  for (int m = 16; m >= N; m >>= 1) {
+    v.lo ^= shfl_xor64(v.lo, m);
+    v.hi ^= shfl_xor64(v.hi, m);
+  }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l < N) red[w][l] = v;
+  __syncthreads();
+  if ((int)threadIdx.x < N && to(threadIdx.x) >= 0) {
+    f128 x = mk(0, 0);
+    for (int i = 0; i < (int)(blockDim.x >> 5); i++) x = fx(x, red[i][threadIdx.x]);
+    atomic_xor128(out + to(threadIdx.x), x);
+  }
+}
+
 // Merkle-path shift sumcheck (SHA-256 statement): the seven tables of a
 // y-round (ta, te, tb, gz, gxl, gxr, g_other) and the claim's eight word
 // coefficients

@@ -202,6 +202,27 @@ __global__ void __launch_bounds__(256) k_lc_round(f128* comb, f128* zv, int len,
   mail_last(mail, out);
 }
 
+// The same round with four lanes a pair (short rounds).
+__global__ void __launch_bounds__(256) k_lc_round_quad(f128* comb, f128* zv, int len, int do_fold, f128 r, int emit,
+                                                       f128* out, MailArgs mail) {
+  const int h = len >> 1, t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 2, q = t & 3;
+  f128 v = mk(0, 0);
+  if (i < h) {
+    f128* p = (q < 2 ? comb : zv) + i + (q & 1 ? h : 0);
+    v = *p;
+    if (do_fold) {
+      v = fx(v, fmul(r, fx(p[len], v)));
+      *p = v;
+    }
+  }
+  if (!emit) return;
+  f128 x, y;
+  quad_factors<false>(v, q, x, y);
+  // odd lanes: sum c1 z1 (out[0]); even lanes: sum (c0 + c1)(z0 + z1) (out[1])
+  block_xor_classes<4>(fmul(x, y), out, [](int c) { return c < 2 ? 1 - c : -1; });
+  mail_last(mail, out);
+}
+
 void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_ptr, const uint16_t* bt_row,
              const f128* eq, f128 alpha, f128 beta, int pin, int k, f128* comb, cudaStream_t s) {
   const int parts = k <= (1 << 14) ? 2 : 4;
@@ -227,9 +248,12 @@ void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_
 }
 void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s,
               const MailArgs& mail) {
-  const int threads = std::max(1, len / 2);
+  const int pairs = std::max(1, len / 2);
   count_launch();
-  k_lc_round<<<(threads + 255) / 256, 256, 0, s>>>(comb, zv, len, fold, r, emit, out, mail);
+  if (pairs <= kQuadPairs)
+    k_lc_round_quad<<<(4 * pairs + 255) / 256, 256, 0, s>>>(comb, zv, len, fold, r, emit, out, mail);
+  else
+    k_lc_round<<<(pairs + 255) / 256, 256, 0, s>>>(comb, zv, len, fold, r, emit, out, mail);
 }
 
 // ------------------------------------------------------------------ K7 --
@@ -248,16 +272,15 @@ __global__ void __launch_bounds__(256) k_lig_msg(const f128* __restrict__ f, con
 }
 
 // fold f and b at r (LSB binding), then emit the next message on the folded
-// pair; TAB: products by r go through a CTA-resident 8-bit window table
-template <bool TAB>
+// pair; products by r go through a CTA-resident 8-bit window table
 __global__ void __launch_bounds__(256) k_lig_fold_msg(const f128* __restrict__ f, const f128* __restrict__ b,
                                                       f128* __restrict__ fo, f128* __restrict__ bo, f128 r,
                                                       size_t n_pairs_out, int emit, f128* __restrict__ out,
                                                       MailArgs mail) {
   extern __shared__ __align__(16) uint8_t sm[];
   MulTab8* rt = reinterpret_cast<MulTab8*>(sm);
-  if (TAB) multab_build(rt, r);
-  auto mr = [&](f128 v) { return TAB ? multab_mul(rt, v) : fmul(r, v); };
+  multab_build(rt, r);
+  auto mr = [&](f128 v) { return multab_mul(rt, v); };
   u256 u0 = zero256(), u2 = zero256();
   for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_pairs_out; j += (size_t)gridDim.x * blockDim.x) {
     f128 fv[4], bv[4];
@@ -277,6 +300,28 @@ __global__ void __launch_bounds__(256) k_lig_fold_msg(const f128* __restrict__ f
     block_xor_out(reduce(u2), out + 1);
     mail_last(mail, out);
   }
+}
+
+// The same for short rounds: four lanes a pair, products by r without a table
+// (building it takes longer than the folds).
+__global__ void __launch_bounds__(256) k_lig_fold_quad(const f128* __restrict__ f, const f128* __restrict__ b,
+                                                       f128* __restrict__ fo, f128* __restrict__ bo, f128 r,
+                                                       int n_pairs_out, int emit, f128* __restrict__ out,
+                                                       MailArgs mail) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j = t >> 2, q = t & 3;
+  f128 v = mk(0, 0);
+  if (j < n_pairs_out) {
+    const f128* p = (q < 2 ? f : b) + 4 * (size_t)j + 2 * (q & 1);
+    v = ld(p);
+    v = fx(v, fmul(r, fx(v, ld(p + 1))));
+    st((q < 2 ? fo : bo) + 2 * (size_t)j + (q & 1), v);
+  }
+  if (!emit) return;
+  f128 x, y;
+  quad_factors<true>(v, q, x, y);
+  // even lanes: sum f0 b0 (out[0]); odd lanes: sum (f0 + f1)(b0 + b1) (out[1])
+  block_xor_classes<4>(fmul(x, y), out, [](int c) { return c < 2 ? c : -1; });
+  mail_last(mail, out);
 }
 
 // Degree-3 sumcheck round over plain F128 vectors (the zerocheck round of
@@ -334,14 +379,14 @@ void lig_msg(const f128* f, const f128* b, size_t n_pairs, f128* out, int sms, c
 void lig_fold_msg(const f128* f, const f128* b, f128* fo, f128* bo, f128 r, size_t n_pairs_out, bool emit, f128* out,
                   int sms, cudaStream_t s, const MailArgs& mail) {
   count_launch();
-  if (n_pairs_out >= (1u << 14)) {
+  if (n_pairs_out > (size_t)kQuadPairs) {
     size_t smem = sizeof(MulTab8);
-    CK(cudaFuncSetAttribute(k_lig_fold_msg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int grid = resident_grid((const void*)k_lig_fold_msg<true>, 256, smem, sms);
-    k_lig_fold_msg<true><<<grid, 256, smem, s>>>(f, b, fo, bo, r, n_pairs_out, emit, out, mail);
+    CK(cudaFuncSetAttribute(k_lig_fold_msg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int grid = resident_grid((const void*)k_lig_fold_msg, 256, smem, sms);
+    k_lig_fold_msg<<<grid, 256, smem, s>>>(f, b, fo, bo, r, n_pairs_out, emit, out, mail);
   } else {
-    const int grid = resident_grid((const void*)k_lig_fold_msg<false>, 256, 0, sms);
-    k_lig_fold_msg<false><<<grid, 256, 0, s>>>(f, b, fo, bo, r, n_pairs_out, emit, out, mail);
+    const unsigned grid = std::max(1u, ((unsigned)n_pairs_out * 4 + 255) / 256);
+    k_lig_fold_quad<<<grid, 256, 0, s>>>(f, b, fo, bo, r, (int)n_pairs_out, emit, out, mail);
   }
 }
 void eq_build(const EqTable* tabs, int count, cudaStream_t s) {

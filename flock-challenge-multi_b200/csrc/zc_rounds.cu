@@ -78,9 +78,7 @@ __device__ __forceinline__ void xshfl(f128& v, int m) {
   v.hi ^= shfl_xor64(v.hi, m);
 }
 
-// MODE 0: packed message round; 1: packed fold + message; 2: fold + message,
-// the fold through a window table of rho; 3: the same through plain products
-// (short rounds, where building the table takes longer than the folds)
+// MODE 0: packed message round; 1: packed fold + message; 2: fold + message
 template <int MODE>
 __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
   extern __shared__ __align__(16) uint8_t smraw[];
@@ -93,12 +91,12 @@ __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
       if (MODE == 1) st(lag + 2048 + i, fmul(A.rho, v));
     }
     __syncthreads();
-  } else if (MODE == 2) {
+  } else {
     multab_build(rt, A.rho);
   }
   auto fold = [&](f128 lo, f128 hi) {
     const f128 d = fx(lo, hi);
-    return fx(lo, MODE == 2 ? multab_mul(rt, d) : fmul(A.rho, d));
+    return fx(lo, multab_mul(rt, d));
   };
   for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < A.halve_n; j += (size_t)gridDim.x * blockDim.x)
     st(A.halve_out + j, fx(ldg(A.etab + 2 * j), ldg(A.etab + 2 * j + 1)));
@@ -182,6 +180,28 @@ __global__ void __launch_bounds__(256, 2) k_zc_round(ZcArgs A) {
   }
   mail_last(A.mail, A.out);
 }
+
+// The fold + message round for few pairs (ns = 0): four lanes a pair, products
+// by rho without a table, each pair weighted by itself.
+__global__ void __launch_bounds__(256) k_zc_round_quad(ZcArgs A) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, j = t >> 2;
+  for (size_t i = t; i < A.halve_n; i += (size_t)gridDim.x * blockDim.x)
+    st(A.halve_out + i, fx(ldg(A.etab + 2 * i), ldg(A.etab + 2 * i + 1)));
+  const int q = t & 3;
+  f128 v = mk(0, 0), w = mk(0, 0);
+  if (j < A.n_pairs) {
+    const f128* p = (q < 2 ? A.a_in : A.b_in) + 4 * (size_t)j + 2 * (q & 1);
+    v = ldg(p);
+    v = fx(v, fmul(A.rho, fx(v, ldg(p + 1))));
+    st((q < 2 ? A.a_out : A.b_out) + 2 * (size_t)j + (q & 1), v);
+    w = mul_xk(ldg(A.etab + (j >> A.nm)), (int)(j & ((1u << A.nm) - 1)) << A.msh);
+  }
+  f128 x, y;
+  quad_factors<false>(v, q, x, y);
+  // odd lanes: sum a1 b1 (out[0]); even lanes: sum (a0 + a1)(b0 + b1) (out[1])
+  block_xor_classes<4>(fmul(fmul(x, y), w), A.out, [](int c) { return c < 2 ? 1 - c : -1; });
+  mail_last(A.mail, A.out);
+}
 }  // namespace
 
 // One zerocheck round launch: out[2 js + {0, 1}] ^= (T1, Tinf)(js) for js < 2^ns.
@@ -201,12 +221,16 @@ void zc_round(int mode, const f128* a_in, const f128* b_in, f128* a_out, f128* b
   A.etab = etab; A.out = out;
   A.halve_out = halve_out; A.halve_n = halve_n;
   A.mail = mail;
-  // the window table pays from about 2^14 folded pairs on (k_lig_fold_msg's line too)
-  const bool plain = mode == 2 && n_pairs < ((size_t)1 << 14);
-  const size_t smem = mode == 0 ? 2048 * sizeof(f128) : mode == 1 ? 4096 * sizeof(f128) : plain ? 0 : sizeof(MulTab8);
-  auto* fn = mode == 0 ? k_zc_round<0> : mode == 1 ? k_zc_round<1> : plain ? k_zc_round<3> : k_zc_round<2>;
+  const bool quad = mode == 2 && ns == 0 && n_pairs <= (size_t)kQuadPairs;
+  const size_t smem = mode == 0 ? 2048 * sizeof(f128) : mode == 1 ? 4096 * sizeof(f128) : quad ? 0 : sizeof(MulTab8);
+  auto* fn = mode == 0 ? k_zc_round<0> : mode == 1 ? k_zc_round<1> : quad ? k_zc_round_quad : k_zc_round<2>;
   if (smem) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const size_t full = (size_t)resident_grid((const void*)fn, 256, smem, sms);
+  if (quad) {
+    count_launch();
+    k_zc_round_quad<<<(unsigned)((4 * n_pairs + 255) / 256), 256, 0, s>>>(A);
+    return;
+  }
   // passes of the wave over the items, each 2^nl pairs (two products and the
   // folds) and one weighting (two products)
   size_t best = ~(size_t)0;
