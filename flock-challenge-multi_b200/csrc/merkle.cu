@@ -13,6 +13,7 @@
 #include "host.hpp"
 #include <emmintrin.h>
 #include <algorithm>
+#include <thread>
 
 namespace {
 // non-root chaining value of one leaf of leaf_size <= 1024 bytes (a single
@@ -377,6 +378,7 @@ uint32_t mail_word(const Mailbox& m, size_t i, cudaStream_t s) {
     const uint64_t w = m.words[i];
     if ((uint32_t)(w >> 32) == m.seq) return (uint32_t)w;
     _mm_pause();
+    if (k % (1u << 9) == 0) std::this_thread::yield();  // more waiting proofs than cores
     if (k % (1u << 14)) continue;
     const cudaError_t e = cudaStreamQuery(s);
     if (e == cudaErrorNotReady) continue;

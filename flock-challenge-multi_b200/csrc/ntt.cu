@@ -503,13 +503,13 @@ __global__ void __launch_bounds__(256, 2) k_ntt_pass_batch(const BatchJob* __res
 
 // The same for the jobs whose pass runs on the tensor cores.
 __global__ void __launch_bounds__(128, 4) k_ntt_pass_batch_t(const BatchJob* __restrict__ jobs, int n_jobs, int pass,
-                                                             uint64_t total_tiles, int max_R, TmShifts sh,
+                                                             uint64_t total_tiles, uint64_t per, int max_R, TmShifts sh,
                                                              unsigned* __restrict__ timeouts) {
   extern __shared__ __align__(16) uint8_t raw[];
   TmapSetup S(raw, max_R);
   uint64_t seq_hi = ~0ull;
   int job = -1;
-  const uint64_t t0 = total_tiles * blockIdx.x / gridDim.x, t1 = total_tiles * (blockIdx.x + 1) / gridDim.x;
+  const uint64_t t0 = blockIdx.x * per, t1 = min(t0 + per, total_tiles);
   for (uint64_t t = t0; t < t1; t++) {
     int lo = 0, hi = n_jobs - 1;
     while (lo < hi) {
@@ -789,6 +789,14 @@ std::vector<NttPass> candidate_shapes_w(int lanes, int l0, int R) {
   return out;
 }
 
+// successive tiles per CTA of a tensor-core pass: enough to share their
+// twiddles and hide the CTA's start, few enough that other streams' kernels
+// find free SMs soon (a batch's commits run beside other proofs' rounds; CTAs
+// that strode over all of a pass held every SM for milliseconds)
+uint64_t tiles_per_cta(uint64_t tiles, int sms) {
+  return std::max<uint64_t>(1, std::min<uint64_t>(8, tiles / ((uint64_t)sms * 4)));
+}
+
 template <bool TR>
 void launch_pass_w(const NttPass& ps, const PassArgs& a, uint64_t tiles, cudaStream_t s) {
   auto k = ps.kind == 1 ? k_ntt_pass_w<TR, 1> : k_ntt_pass_w<TR, 2>;
@@ -809,9 +817,7 @@ void launch_pass(const NttPass& ps, f128* data, const f128* ev, int log_d, int l
   if (ps.kind == 3) {
     if (transpose) throw CudaError("ntt: tensor passes run forward only");
     CK(cudaFuncSetAttribute(k_ntt_pass_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_t_smem(kMaxRt)));
-    // successive tiles per CTA: enough to share their twiddles and hide the
-    // CTA's start, few enough that other streams' kernels find free SMs soon
-    const uint64_t per = std::max<uint64_t>(1, std::min<uint64_t>(8, tiles / (148 * 4)));
+    const uint64_t per = tiles_per_cta(tiles, 148);
     count_launch();
     k_ntt_pass_t<<<(unsigned)((tiles + per - 1) / per), 128, pass_t_smem(ps.R), s>>>(a, tiles, per, tm_shifts(),
                                                                                     device_timeouts().dev);
@@ -946,10 +952,10 @@ void ntt_pass_batch_t(const BatchJob* jobs, int n_jobs, int pass, uint64_t total
                       cudaStream_t s) {
   const size_t smem = pass_t_smem(max_R);
   CK(cudaFuncSetAttribute(k_ntt_pass_batch_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_t_smem(kMaxRt)));
-  const uint64_t grid = (uint64_t)resident_grid((const void*)k_ntt_pass_batch_t, 128, smem, sms);
+  const uint64_t per = tiles_per_cta(total_tiles, sms);
   count_launch();
-  k_ntt_pass_batch_t<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(grid, total_tiles)), 128, smem, s>>>(
-      jobs, n_jobs, pass, total_tiles, max_R, tm_shifts(), device_timeouts().dev);
+  k_ntt_pass_batch_t<<<(unsigned)((total_tiles + per - 1) / per), 128, smem, s>>>(
+      jobs, n_jobs, pass, total_tiles, per, max_R, tm_shifts(), device_timeouts().dev);
 }
 
 NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaStream_t s, double* best_ms) {
