@@ -67,7 +67,7 @@ def algorithmic_bytes(phase: str, log2: int) -> int:
 
 # phase -> (the phase's kernels, launches per proof, what the algorithmic bytes count)
 PHASE_KERNEL = {
-    "rs_encode": ("k_ntt_pass_w (4-bit table passes; the first reads the message)", 0,
+    "rs_encode": ("k_ntt_pass_t (tensor-core passes; the first reads the message)", 0,
                   "read the message (2^25 F128), write the codeword (2^26 F128)"),
     "merkle_commit": ("k_merkle_leaves/parents/top", 22, "read the 1 GiB codeword, write 32 B per leaf"),
     "zerocheck_round1": ("k_zc_round1_ab + k_zc_round1_c", 2, "read packed a, b, c (3 x 512 MiB)"),
@@ -412,8 +412,14 @@ def table_product_peak() -> float:
 
 def product_ceiling(plan_desc: str) -> tuple:
     """(ceiling, definition) of the GF(2^128) product as the tuned plan's
-    passes compute it: integer multiplies, table lookups, or both pipes at
-    once (the mixed passes send half of the lanes each way)."""
+    passes compute it: bit matrices on the tensor cores, integer multiplies,
+    table lookups, or the last two at once (the mixed passes send half of the
+    lanes each way)."""
+    if "/mma" in plan_desc:
+        # spreading a value's bits and merging its counts: 28 shifts and 32
+        # masks, 36 selects and 13 XORs and shifts, 64 a clock per SM
+        return 148 * sm_mhz() * 1e6 * 64 / 109, ("tensor cores: bounded by the integer pipe, 148 SMs x max SM clock x "
+                                                "64 / 109 operations to spread and merge a product's bits")
     if "/tab+imad" in plan_desc:
         return 2 * min(int_product_peak(), table_product_peak()), "mixed: both pipes, half of the products each"
     if "/tab" in plan_desc:
@@ -689,7 +695,9 @@ def run_ours(args, world, rank, local):
     kname, klaunches, kdesc = PHASE_KERNEL[dom]
     if dom == "rs_encode":  # one launch per pass of the tuned plan
         klaunches = plan_desc.count(" + ") + 1
-        if "/tab" not in plan_desc:
+        if "/tab" in plan_desc:
+            kname = "k_ntt_pass_w (4-bit table passes; the first reads the message)"
+        elif "/mma" not in plan_desc:
             kname = "k_ntt_pass (integer products; the first pass reads the message)"
     kbytes = algorithmic_bytes(dom, log2)
     # the phase's events bracket only its own launches on the prover stream:

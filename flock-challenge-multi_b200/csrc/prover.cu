@@ -208,8 +208,8 @@ void Setup::capture_commit() {
 }
 
 // Fused witness + RS encode + Merkle commit of several seeded proofs: every
-// stage is one launch over all jobs (persistent NTT passes over the tiles of
-// every job, one parent level of every tree per launch), captured as one
+// stage is one launch over all jobs (each NTT pass covers the tiles of every
+// job, each parent level that of every tree), captured as one
 // CUDA graph and launched on `st`.  The setups' streams wait for it; each
 // proof then continues with Setup::prove(..., committed = true).  The call
 // returns once the work is queued; release the handle after `st` finished.

@@ -522,7 +522,7 @@ int flock_poll(flock_ctx* ctx, uint64_t ticket, flock_result* res, int timeout_m
  * admitted in order, in waves of as many as fit the context's HBM budget.
  * The witnesses, RS encodes and Merkle trees of a wave's seeded jobs run in
  * groups of 8 jobs, each group as one CUDA graph of fused launches over its
- * jobs (one persistent NTT pass kernel over the tiles of every job, one tree
+ * jobs (one kernel per NTT pass over the tiles of every job, one tree
  * level of every job per launch); the remaining phases of each proof run
  * concurrently on `threads` host threads, one CUDA stream each, starting as
  * soon as the proof's group is queued.  Every result is
