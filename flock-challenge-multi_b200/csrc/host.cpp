@@ -147,11 +147,6 @@ std::vector<f128> transpose128(const std::vector<f128>& rows) {
   return out;
 }
 
-void subset_sums8(const f128* v8, f128* out) {
-  out[0] = mk(0, 0);
-  for (int v = 1; v < 256; v++) out[v] = fx(out[v & (v - 1)], v8[__builtin_ctz(v)]);
-}
-
 // --------------------------------------------------------------- BLAKE3 --
 const uint32_t kB3IV[8] = {0x6A09E667u, 0xBB67AE85u, 0x3C6EF372u, 0xA54FF53Au,
                                 0x510E527Fu, 0x9B05688Cu, 0x1F83D9ABu, 0x5BE0CD19u};

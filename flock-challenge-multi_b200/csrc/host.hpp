@@ -24,8 +24,6 @@ std::vector<f128> hlagrange(f128 z, int node_base);           // 64 weights over
 void transpose64(uint64_t a[64]);
 // 128 x 128 bit transpose: bit i of out[j] = bit j of rows[i] (128 rows)
 std::vector<f128> transpose128(const std::vector<f128>& rows);
-// out[v] = XOR of v8[j] over the set bits j of v, v < 256
-void subset_sums8(const f128* v8, f128* out);
 uint8_t hgf8_mul(uint8_t a, uint8_t b);
 
 // ---- BLAKE3 hasher (incremental, root / XOF) ----

@@ -319,6 +319,8 @@ struct EqTable {
 constexpr int kMaxEqTables = 4;
 void eq_build(const EqTable* tabs, int count, cudaStream_t s);  // one launch
 void eq_build(const f128* r, int n, f128 scale, f128* out, cudaStream_t s);
+// out[256 g + v] = XOR of basis[8 g + j] over the set bits j of v, g < groups <= 32 (basis: host)
+void subset_tables(const f128* basis, int groups, f128* out, cudaStream_t s);
 void outer64(const f128* L, const f128* e, size_t n_e, f128* out, cudaStream_t s);
 void inner(const f128* f, const f128* g, size_t n, f128* out, int grid, cudaStream_t s, const MailArgs& mail = {});
 size_t round1_tables_size();

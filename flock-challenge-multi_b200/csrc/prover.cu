@@ -543,10 +543,11 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     CK(cudaMemsetAsync(out, 0, 1024 * sizeof(f128), st));
     size_t n_blocks128 = (size_t)1 << (m - 13);
     zc_round1(a, b, z, tabs_r1, scratch_eq(), n_blocks128, out, gs, st);
-    fetch(out, 1024, h_out);
+    CK(cudaMemcpyAsync(h_out, out, 1024 * sizeof(f128), cudaMemcpyDeviceToHost, st));
     // from here on `out` is a ring of 128 zeroed 8-value slots: every round
     // message accumulates into a fresh slot, so no round needs its own clear
     CK(cudaMemsetAsync(out, 0, 1024 * sizeof(f128), st));
+    CK(cudaStreamSynchronize(st));
     // P_AB(l) = sum_k phi8(e_k) H(l, k)
     const f128* phi8 = phi8_table();
     P.r1_ab.assign(64, mk(0, 0));
@@ -579,9 +580,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   f128 zc_z = tr.sample();
   {
     std::vector<f128> L = hlagrange(zc_z, 0);
-    std::vector<f128> lagt(8 * 256);
-    for (int k = 0; k < 8; k++) subset_sums8(L.data() + 8 * k, lagt.data() + k * 256);
-    CK(cudaMemcpyAsync(lag, lagt.data(), lagt.size() * sizeof(f128), cudaMemcpyHostToDevice, st));
+    subset_tables(L.data(), 8, lag, st);
     std::vector<f128> LL = hlagrange(zc_z, 64);
     f128 ce = mk(0, 0);
     for (int i = 0; i < 64; i++) ce = fx(ce, hmul(LL[i], P.r1_c[i]));
@@ -613,6 +612,19 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   const f128 C_inv = hinv(C_full);
   const f128* etab = scratch_eq();
   size_t etab_len = (size_t)1 << (m - 13), etab_off = etab_len;
+  // The last rounds' vectors are small.  Once a round has at most
+  // kHostZcPairs pairs and only the random suffix weights its pairs (round 7
+  // on), the remaining rounds run on the host from one copy of the vectors
+  // and the eq table: the same folds and sums, without a GPU round trip per
+  // round (a 512-pair round is about 4 K host products, 20 us).  The copies go
+  // to pinned memory (the openings' staging area, unused so far) right behind
+  // the round that leaves the vectors, while the host reads its message: zerocheck
+  // rounds of a 2^10 proof 0.331 -> 0.285 ms. Three
+  // copies into pageable memory after the message had each been waited for.
+  constexpr size_t kHostZcPairs = 512;
+  static_assert(9 * kHostZcPairs * sizeof(f128) <= kStageBytes, "the tail's vectors fit the staging area");
+  f128* const h_tail = reinterpret_cast<f128*>(h_stage);
+  auto host_next = [&](int round, size_t n_pairs) { return round >= 7 && n_pairs > 0 && n_pairs <= kHostZcPairs; };
   auto run_round = [&](int k, int mode, const f128* ain, const f128* bin, f128* aout, f128* bout, f128 rho,
                        size_t n_pairs) {
     const int st0 = 7 + k;
@@ -645,6 +657,12 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
       etab_len = nxt_len;
       etab_off += nxt_len;
     }
+    if (host_next(k + 1, n_pairs / 2)) {  // its vectors follow the message to the host
+      const size_t n = n_pairs / 2;
+      CK(cudaMemcpyAsync(h_tail, aout, 4 * n * sizeof(f128), cudaMemcpyDeviceToHost, st));
+      CK(cudaMemcpyAsync(h_tail + 4 * n, bout, 4 * n * sizeof(f128), cudaMemcpyDeviceToHost, st));
+      CK(cudaMemcpyAsync(h_tail + 8 * n, etab, n * sizeof(f128), cudaMemcpyDeviceToHost, st));
+    }
     mailbox_read(mail, h_out, 8, st);
     f128 g1 = mk(0, 0), gi = mk(0, 0);
     for (int js = 0; js < (1 << ns); js++) {
@@ -654,12 +672,6 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     h_out[0] = g1;
     h_out[1] = gi;
   };
-  // The last rounds' vectors are small.  Once a round has at most
-  // kHostZcPairs pairs and only the random suffix weights its pairs (round 7
-  // on), the remaining rounds run on the host from one copy of the vectors
-  // and the eq table: the same folds and sums, without a GPU round trip per
-  // round (a 512-pair round is about 4 K host products, 20 us).
-  constexpr size_t kHostZcPairs = 512;
   bool host_tail = false;
   std::vector<f128> ha, hb, he;  // the vectors and eq table once on the host
   auto host_round = [&](f128 rho) {
@@ -697,15 +709,12 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     rhos.push_back(rho);
     if (i < n_mlv - 1) {
       size_t n_pairs_out = (size_t)1 << (n_mlv - i - 2);
-      if (!host_tail && i + 1 >= 7 && n_pairs_out <= kHostZcPairs) {
-        // av, bv hold the 4 n values the round folds; etab its n eq weights
-        ha.resize(4 * n_pairs_out);
-        hb.resize(4 * n_pairs_out);
-        he.resize(n_pairs_out);
-        CK(cudaMemcpyAsync(ha.data(), av, ha.size() * sizeof(f128), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(hb.data(), bv, hb.size() * sizeof(f128), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(he.data(), etab, he.size() * sizeof(f128), cudaMemcpyDeviceToHost, st));
+      if (!host_tail && host_next(i + 1, n_pairs_out)) {
+        // the 4 n values of a and b that the round folds, and its n eq weights
         CK(cudaStreamSynchronize(st));
+        ha.assign(h_tail, h_tail + 4 * n_pairs_out);
+        hb.assign(h_tail + 4 * n_pairs_out, h_tail + 8 * n_pairs_out);
+        he.assign(h_tail + 8 * n_pairs_out, h_tail + 9 * n_pairs_out);
         host_tail = true;
       }
       if (host_tail) host_round(rho);
@@ -960,13 +969,10 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     target = fx(target, hmul(gpd, pd_value));
   }
   {
-    std::vector<f128> T(2 * 16 * 256);
-    for (int k = 0; k < 2; k++) {
-      std::vector<f128> sc(128);
-      for (int bb = 0; bb < 128; bb++) sc[bb] = hmul(gam[k], eqdd[k][bb]);
-      for (int byte = 0; byte < 16; byte++) subset_sums8(sc.data() + 8 * byte, T.data() + (size_t)k * 4096 + byte * 256);
-    }
-    CK(cudaMemcpyAsync(bc_tabs, T.data(), T.size() * sizeof(f128), cudaMemcpyHostToDevice, st));
+    f128 sc[256];
+    for (int k = 0; k < 2; k++)
+      for (int bb = 0; bb < 128; bb++) sc[128 * k + bb] = hmul(gam[k], eqdd[k][bb]);
+    subset_tables(sc, 32, bc_tabs, st);
     // eq(suffix_k, i) = lo_k(i mod 2^lo_bits) * hi_k(i >> lo_bits), both tables
     // on the device; chunks of up to 2^14 values (each CTA builds its two
     // product tables once per chunk), as long as the four tables fit eqbuf,

@@ -91,6 +91,25 @@ __global__ void k_outer64(Vec64 L, const f128* __restrict__ e, size_t n_e, f128*
   st(out + i, fmul(L.v[i & 63], ldg(e + (i >> 6))));
 }
 
+// The byte tables of a GF(2)-linear map, group g's basis values in the launch's
+// parameters: eight selected XORs a value, one CTA a group, bound by the
+// launch.  Built on the host, the 128 KiB of the ring switch's tables took a
+// 2^10-compression proof more than 15 us (8192 XORs, fresh pages, a copy from
+// pageable memory): its proof gained 15 us.
+struct SubsetBasis {
+  f128 v[256];
+};
+__global__ void k_subset_tables(const __grid_constant__ SubsetBasis B, f128* __restrict__ out) {
+  const unsigned g = blockIdx.x, v = threadIdx.x;
+  f128 x = mk(0, 0);
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const f128 y = B.v[8 * g + j];
+    if (v >> j & 1) x = fx(x, y);
+  }
+  st(out + 256 * g + v, x);
+}
+
 // out[i] += beta * x[i]
 __global__ void k_axpy(f128* __restrict__ out, const f128* __restrict__ x, f128 beta, size_t n) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -417,6 +436,13 @@ void outer64(const f128* L, const f128* e, size_t n_e, f128* out, cudaStream_t s
   for (int j = 0; j < 64; j++) V.v[j] = L[j];
   count_launch();
   k_outer64<<<(unsigned)((64 * n_e + 255) / 256), 256, 0, s>>>(V, e, n_e, out);
+}
+void subset_tables(const f128* basis, int groups, f128* out, cudaStream_t s) {
+  if (groups < 1 || groups > 32) throw CudaError("subset_tables: 1 to 32 groups");
+  SubsetBasis B;
+  for (int i = 0; i < 256; i++) B.v[i] = i < 8 * groups ? basis[i] : mk(0, 0);
+  count_launch();
+  k_subset_tables<<<(unsigned)groups, 256, 0, s>>>(B, out);
 }
 void axpy(f128* out, const f128* x, f128 beta, size_t n, cudaStream_t s) {
   count_launch(); k_axpy<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, x, beta, n);
