@@ -118,7 +118,7 @@ size_t ceil_log2(size_t n);
 // phi8(0xF7), phi8(0x53), phi8(0xB5) and gamma^(2^i) / (1 + gamma^(2^i)),
 // gamma = x, i = 1, 2, 4, 8 as shifts
 std::vector<f128> small_consts();
-std::vector<f128> medium_consts();
+const std::vector<f128>& medium_consts();
 
 // ---- R1CS statements: one compression per 2^k_log-bit block ----
 // The hash a statement encodes.  BLAKE3 (r1cs_hashes/blake3.rs): 2^14-bit
@@ -180,7 +180,14 @@ const Ladder* ladder_for(int m);
 
 // ---- proof object + FLOCK v4 bincode-fixint writer (proof_io.rs:40-215) ----
 using H32 = std::array<uint8_t, 32>;
-struct Opening { std::vector<std::vector<f128>> rows; std::vector<H32> proof; };
+struct Opening {
+  std::vector<std::vector<f128>> rows;
+  std::vector<H32> proof;
+  // a prover's opening instead, as it lies in its staging area until the next
+  // proof: nq rows of `lanes` values, then ns hashes
+  const uint8_t* staged = nullptr;
+  size_t nq = 0, lanes = 0, ns = 0;
+};
 struct Proof {
   H32 root{};
   uint64_t m = 0;

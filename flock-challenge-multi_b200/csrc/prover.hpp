@@ -170,7 +170,7 @@ class Setup {
   uint64_t grind(Transcript& tr, uint32_t bits);
   std::vector<size_t> sample_queries(Transcript& tr, size_t block_len, size_t count);
   // queues the opening's gathers and its copy into the pinned staging area;
-  // `o` is filled by finish_openings once the stream has finished
+  // finish_openings points `o` at it once the stream has finished
   void open(Opening& o, const f128* cw, const uint32_t* tree, size_t n_leaves, int lanes, const std::vector<size_t>& q);
   void finish_openings();
   struct PendingOpen {
@@ -184,7 +184,8 @@ class Setup {
   void mark(int phase);
   f128* scratch_eq() { return eqbuf[0]; }
 
-  uint8_t lde_m[64][64] = {};  // GF(2^8) extension S -> Lambda (Lagrange basis)
+  // the GF(2^8) extension S -> Lambda: bit s % 8 of [l][k][s / 8] is bit k of L_s(64 + l)
+  uint8_t lde_bits[64][8][8] = {};
   const Ladder* lad = nullptr;
   std::array<uint8_t, 32> digest{};
   f128 *z = nullptr, *a = nullptr, *b = nullptr, *cw0 = nullptr;
