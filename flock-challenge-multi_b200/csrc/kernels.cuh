@@ -288,7 +288,8 @@ void merkle_parents_batch(const BatchJob* jobs, int n_jobs, int level, uint64_t 
 void merkle_top_batch(const BatchJob* jobs, int n_jobs, cudaStream_t s);
 
 // K2 / K9
-void merkle_build(const void* data, size_t n_leaves, size_t leaf_size, uint32_t* tree, cudaStream_t s);
+void merkle_build(const void* data, size_t n_leaves, size_t leaf_size, uint32_t* tree, cudaStream_t s,
+                  const MailArgs& mail = {});  // mail: for the root, of at least two leaves
 void merkle_leaves(const void* data, size_t n_leaves, size_t leaf_size, uint32_t* out, cudaStream_t s);
 // the same over the Merkle hash fn (0 SHA-256: leaf SHA256(bytes), parent
 // SHA256(l || r), leaf sizes multiples of 4 bytes; 1 BLAKE3: the above)
@@ -338,7 +339,8 @@ void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv
 void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s,
               const MailArgs& mail = {});
 // s_hat_v of the ab claim from the block-folded z (2^k_log values)
-void ring_shat_ab(const f128* zv_pre, const f128* eqt, int k_log, f128* out, cudaStream_t s);
+void ring_shat_ab(const f128* zv_pre, const f128* eqt, int k_log, f128* out, cudaStream_t s,
+                  const MailArgs& mail = {});
 // f, msg (optional): also XOR the first Ligerito message over (f, b_combined)
 // into msg[0..2) (zeroed), the values k_lig_msg gives for the same pairs
 void ring_bcombined_ct(const f128* elo0, const f128* ehi0, const f128* elo1, const f128* ehi1, const f128* L0,

@@ -155,8 +155,10 @@ __global__ void k_merkle_parents(const uint32_t* __restrict__ in, uint32_t* __re
   parent_cv(in + 16 * i, out + 8 * i);
 }
 
-__global__ void k_merkle_top(uint32_t* tree, size_t level_start, size_t level_len) {
+__global__ void k_merkle_top(uint32_t* tree, size_t level_start, size_t level_len, MailArgs M) {
   tree_top(tree, level_start, level_len);
+  if (M.words && threadIdx.x < 8)  // the root, visible to the CTA after tree_top's last barrier
+    M.words[threadIdx.x] = (uint64_t)M.seq << 32 | tree[8 * (level_start + 2 * level_len - 2) + threadIdx.x];
 }
 
 void merkle_leaves_batch(const BatchJob* jobs, int n_jobs, uint64_t total, cudaStream_t s) {
@@ -231,7 +233,7 @@ void merkle_leaves(const void* data, size_t n_leaves, size_t leaf_size, uint32_t
 }
 
 void merkle_build(const void* data, size_t n_leaves, size_t leaf_size, uint32_t* tree, int fn, cudaStream_t s) {
-  if (fn != flock::kFnSha256) return merkle_build(data, n_leaves, leaf_size, tree, s);
+  if (fn != flock::kFnSha256) return merkle_build(data, n_leaves, leaf_size, tree, s, MailArgs{});
   merkle_leaves(data, n_leaves, leaf_size, tree, fn, s);
   for (size_t start = 0, len = n_leaves; len > 1; start += len, len >>= 1) {
     const size_t n = len >> 1;
@@ -240,7 +242,8 @@ void merkle_build(const void* data, size_t n_leaves, size_t leaf_size, uint32_t*
   }
 }
 
-void merkle_build(const void* data, size_t n_leaves, size_t leaf_size, uint32_t* tree, cudaStream_t s) {
+void merkle_build(const void* data, size_t n_leaves, size_t leaf_size, uint32_t* tree, cudaStream_t s,
+                  const MailArgs& mail) {
   count_launch(); k_merkle_leaves<<<(unsigned)((n_leaves + 127) / 128), 128, 0, s>>>((const uint8_t*)data, leaf_size, n_leaves, tree);
   size_t start = 0, len = n_leaves;
   while (len > 1024) {
@@ -249,7 +252,7 @@ void merkle_build(const void* data, size_t n_leaves, size_t leaf_size, uint32_t*
     start += len;
     len = n;
   }
-  if (len > 1) count_launch(), k_merkle_top<<<1, 512, 0, s>>>(tree, start, len);
+  if (len > 1) count_launch(), k_merkle_top<<<1, 512, 0, s>>>(tree, start, len, mail);
 }
 
 std::vector<uint64_t> multiproof_ids(const std::vector<size_t>& q, size_t n_leaves) {
@@ -298,11 +301,23 @@ void scatter(f128* dst, const uint64_t* pos, const f128* vals, size_t n, cudaStr
 }  // namespace flock
 
 // ---------------------------------------------------------------- PoW --
-__global__ void k_pow(uint4 d0, uint4 d1, uint32_t bits, uint64_t start, uint64_t count,
-                      unsigned long long* __restrict__ found) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  uint64_t n = start + i;
+// The CTA of a range that finishes last posts the smallest valid nonce (or ~0)
+// and readies its word for the next range; every thread calls it.  A launch of
+// its own for the post waited 1.5 us behind the search and took 2.
+__device__ __forceinline__ void post_found(const MailArgs& M, unsigned long long* found) {
+  if (!M.words) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x || atomicAdd(M.ticket, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  const unsigned long long v = atomicExch(found, ~0ull);
+  M.words[0] = (uint64_t)M.seq << 32 | (uint32_t)v;
+  M.words[1] = (uint64_t)M.seq << 32 | (uint32_t)(v >> 32);
+  *M.ticket = 0;
+}
+
+__device__ __forceinline__ void pow_try(const uint4& d0, const uint4& d1, uint32_t bits, uint64_t n,
+                                        unsigned long long* found) {
   if (n >= *found) return;
   uint32_t m[16] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w, (uint32_t)n, (uint32_t)(n >> 32), 0, 0, 0, 0, 0, 0};
   uint32_t h[8];
@@ -315,12 +330,16 @@ __global__ void k_pow(uint4 d0, uint4 d1, uint32_t bits, uint64_t start, uint64_
   if (ok) atomicMin(found, (unsigned long long)n);
 }
 
+__global__ void k_pow(uint4 d0, uint4 d1, uint32_t bits, uint64_t start, uint64_t count, unsigned long long* found,
+                      MailArgs M) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < count) pow_try(d0, d1, bits, start + i, found);
+  post_found(M, found);
+}
+
 // SHA256(digest || nonce LE), one padded block (challenger.rs:589-595)
-__global__ void k_pow_sha(uint4 d0, uint4 d1, uint32_t bits, uint64_t start, uint64_t count,
-                          unsigned long long* __restrict__ found) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  uint64_t n = start + i;
+__device__ __forceinline__ void pow_try_sha(const uint4& d0, const uint4& d1, uint32_t bits, uint64_t n,
+                                            unsigned long long* found) {
   if (n >= *found) return;
   uint32_t w[16] = {sha_d::bswap(d0.x), sha_d::bswap(d0.y), sha_d::bswap(d0.z), sha_d::bswap(d0.w),
                     sha_d::bswap(d1.x), sha_d::bswap(d1.y), sha_d::bswap(d1.z), sha_d::bswap(d1.w),
@@ -336,6 +355,12 @@ __global__ void k_pow_sha(uint4 d0, uint4 d1, uint32_t bits, uint64_t start, uin
   if (ok && extra) ok = ((((st[full >> 2] >> (24 - 8 * (full & 3))) & 0xFF) >> (8 - extra)) == 0);
   if (ok) atomicMin(found, (unsigned long long)n);
 }
+__global__ void k_pow_sha(uint4 d0, uint4 d1, uint32_t bits, uint64_t start, uint64_t count, unsigned long long* found,
+                          MailArgs M) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < count) pow_try_sha(d0, d1, bits, start + i, found);
+  post_found(M, found);
+}
 
 namespace {
 // One range of the search per call of `scan`, which returns the smallest valid
@@ -350,12 +375,12 @@ uint64_t pow_ranges(const uint8_t digest[32], uint32_t bits, cudaStream_t s, uns
   memcpy(&d1, digest + 16, 16);
   const uint64_t chunk = 1ull << (bits + 1 < 16 ? 16 : bits + 1 > 22 ? 22 : bits + 1);
   for (uint64_t start = 0;; start += chunk) {
-    const uint64_t n = scan([&] {
+    const uint64_t n = scan([&](const MailArgs& mail) {
       count_launch();
       if (fn == flock::kFnSha256)
-        k_pow_sha<<<(unsigned)(chunk / 256), 256, 0, s>>>(d0, d1, bits, start, chunk, d_found);
+        k_pow_sha<<<(unsigned)(chunk / 256), 256, 0, s>>>(d0, d1, bits, start, chunk, d_found, mail);
       else
-        k_pow<<<(unsigned)(chunk / 256), 256, 0, s>>>(d0, d1, bits, start, chunk, d_found);
+        k_pow<<<(unsigned)(chunk / 256), 256, 0, s>>>(d0, d1, bits, start, chunk, d_found, mail);
     });
     if (n != ~0ull) return n;
   }
@@ -364,13 +389,6 @@ uint64_t pow_ranges(const uint8_t digest[32], uint32_t bits, cudaStream_t s, uns
 __global__ void k_mail(const uint32_t* __restrict__ src, int n, volatile uint64_t* words, uint32_t seq) {
   const int t = threadIdx.x;
   if (t < n) words[t] = (uint64_t)seq << 32 | src[t];
-}
-// a search's result, and its word ready for the next search
-__global__ void k_mail_found(unsigned long long* found, volatile uint64_t* words, uint32_t seq) {
-  const unsigned long long v = *found;
-  words[0] = (uint64_t)seq << 32 | (uint32_t)v;
-  words[1] = (uint64_t)seq << 32 | (uint32_t)(v >> 32);
-  *found = ~0ull;
 }
 
 uint32_t mail_word(const Mailbox& m, size_t i, cudaStream_t s) {
@@ -415,7 +433,7 @@ uint64_t pow_search(const uint8_t digest[32], uint32_t bits, cudaStream_t s, uns
   return pow_ranges(digest, bits, s, d_found, fn, [&](auto&& launch) -> uint64_t {
     *h_found = ~0ull;
     CK(cudaMemcpyAsync(d_found, h_found, 8, cudaMemcpyHostToDevice, s));
-    launch();
+    launch(MailArgs{});
     CK(cudaMemcpyAsync(h_found, d_found, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     return *h_found;
@@ -424,10 +442,7 @@ uint64_t pow_search(const uint8_t digest[32], uint32_t bits, cudaStream_t s, uns
 uint64_t pow_search(const uint8_t digest[32], uint32_t bits, cudaStream_t s, unsigned long long* d_found, Mailbox& m,
                     int fn) {
   return pow_ranges(digest, bits, s, d_found, fn, [&](auto&& launch) -> uint64_t {
-    launch();
-    const MailArgs a = m.next(1);
-    count_launch();
-    k_mail_found<<<1, 1, 0, s>>>(d_found, a.words, a.seq);
+    launch(m.next(1));
     const uint64_t lo = mail_word(m, 0, s);
     return lo | (uint64_t)mail_word(m, 1, s) << 32;
   });

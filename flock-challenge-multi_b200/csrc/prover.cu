@@ -958,9 +958,9 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     std::vector<f128> eqt = heq(std::vector<f128>(r_inner_rest.begin() + 1, r_inner_rest.end()));
     CK(cudaMemcpyAsync(eq_inner, eqt.data(), eqt.size() * sizeof(f128), cudaMemcpyHostToDevice, st));
     f128* ro = next_out(16);
-    ring_shat_ab(zv_pre, eq_inner, k_log, ro, st);
+    ring_shat_ab(zv_pre, eq_inner, k_log, ro, st, mail.next(128));
     std::vector<f128> sv(128);
-    fetch(ro, 128, sv.data());
+    mailbox_read(mail, sv.data(), 128, st);
     P.s_hat_v.push_back(sv);
     P.s_hat_v.push_back(s_hat_v_c);
   }
@@ -1126,8 +1126,16 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   // level 1 commit
   auto commit = [&](Level& L) {
     ntt_rs_encode(f, L.cw, L.log_msg_pos, L.lanes, L.rate, st);
-    merkle_build(L.cw, L.positions, (size_t)L.lanes * 16, L.tree, merkle_fn, st);
-    H32 rt = root_of(L.tree, L.positions);
+    H32 rt;
+    if (merkle_fn != kFnSha256 && L.positions > 1) {  // the tree's last kernel posts the root
+      merkle_build(L.cw, L.positions, (size_t)L.lanes * 16, L.tree, st, mail.next(2));
+      f128 v[2];
+      mailbox_read(mail, v, 2, st);
+      memcpy(rt.data(), v, 32);
+    } else {
+      merkle_build(L.cw, L.positions, (size_t)L.lanes * 16, L.tree, merkle_fn, st);
+      rt = root_of(L.tree, L.positions);
+    }
     P.roots.push_back(rt);
     tr.bytes(rt.data(), 32);
   };

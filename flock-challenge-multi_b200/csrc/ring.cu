@@ -21,7 +21,7 @@
 // across the CTA (warp shuffles, then the four warp sums)
 // a thread per 128-bit word of the block (128 to 1024 words), a CTA per bit r
 __global__ void __launch_bounds__(1024) k_shat_from_zvec(const f128* __restrict__ zv, const f128* __restrict__ eqt,
-                                                         f128* __restrict__ out) {
+                                                         f128* __restrict__ out, MailArgs M) {
   __shared__ f128 red[32];
   const int r = blockIdx.x, t = threadIdx.x;
   f128 v = warp_xor(fmul(ldg(eqt + t), ldg(zv + 128 * t + r)));
@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(1024) k_shat_from_zvec(const f128* __restrict_
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) s = fx(s, red[w]);
     out[r] = s;
   }
+  mail_last(M, out);
 }
 
 namespace {
@@ -115,9 +116,9 @@ __global__ void __launch_bounds__(256, 3) k_bcombined_msg(const f128* __restrict
   mail_last(mail, msg);
 }
 
-void ring_shat_ab(const f128* zv_pre, const f128* eqt, int k_log, f128* out, cudaStream_t s) {
+void ring_shat_ab(const f128* zv_pre, const f128* eqt, int k_log, f128* out, cudaStream_t s, const MailArgs& mail) {
   count_launch();
-  k_shat_from_zvec<<<128, 1 << (k_log - 7), 0, s>>>(zv_pre, eqt, out);
+  k_shat_from_zvec<<<128, 1 << (k_log - 7), 0, s>>>(zv_pre, eqt, out, mail);
 }
 
 void ring_bcombined_ct(const f128* elo0, const f128* ehi0, const f128* elo1, const f128* ehi1, const f128* L0,
