@@ -15,6 +15,7 @@ struct flock_ctx {
   int sms = 1;  // the device's SM count
   uint64_t budget = 0;
   cudaStream_t st = nullptr;
+  WaitLimit waits;  // of the kernels that this context's calls launch
   std::string err;
   std::mutex mu;
   std::unique_ptr<flock::Server> server;
@@ -163,6 +164,7 @@ int flock_ctx_create(int device, uint64_t hbm_budget_bytes, flock_ctx** out) {
     CK(cudaSetDevice(device));
     CK(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device));
     CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
+    c->waits.ran_out = device_timeouts().dev;
     return FLOCK_OK;
   });
   if (rc) {
@@ -230,6 +232,18 @@ int flock_ctx_set_transcript(flock_ctx* c, int hash) {
   if (!c || (hash != FLOCK_HASH_SHA256 && hash != FLOCK_HASH_BLAKE3)) return FLOCK_ERR_ARG;
   std::lock_guard<std::mutex> lk(c->vmu);
   c->fs_fn = hash;
+  return FLOCK_OK;
+}
+
+int flock_setup_set_wait_polls(flock_setup* s, uint32_t polls) {
+  if (!s) return FLOCK_ERR_ARG;
+  s->s->waits.polls = polls;
+  return FLOCK_OK;
+}
+
+int flock_ctx_set_wait_polls(flock_ctx* c, uint32_t polls) {
+  if (!c) return FLOCK_ERR_ARG;
+  c->waits.polls = polls;
   return FLOCK_OK;
 }
 
@@ -655,7 +669,7 @@ int flock_pcs_commit(flock_ctx* c, const uint64_t* z_packed, uint32_t m, uint8_t
     CK(cudaMalloc(&pd->tree, (2 * pd->n_leaves - 1) * 32));
     DevBuf<f128> z(n_msg);
     CK(cudaMemcpyAsync(z.p, z_packed, n_msg * sizeof(f128), cudaMemcpyHostToDevice, c->st));
-    ntt_rs_encode(z.p, pd->cw, (int)m - 13, 64, 1, c->st);
+    ntt_rs_encode(z.p, pd->cw, (int)m - 13, 64, 1, c->st, c->waits);
     merkle_build(pd->cw, pd->n_leaves, 64 * sizeof(f128), pd->tree, c->st);
     CK(cudaMemcpyAsync(root32, pd->tree + 8 * (2 * pd->n_leaves - 2), 32, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -1151,7 +1165,7 @@ int flock_ntt_rs_encode(flock_ctx* c, const uint64_t* msg, uint32_t log_msg_pos,
     size_t n = ((size_t)lanes) << log_msg_pos, nc = n << rate;
     DevBuf<f128> dm(n), dc(nc);
     CK(cudaMemcpyAsync(dm.p, msg, n * 16, cudaMemcpyHostToDevice, c->st));
-    ntt_rs_encode(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, c->st);
+    ntt_rs_encode(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, c->st, c->waits);
     CK(cudaMemcpyAsync(out, dc.p, nc * 16, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     check_device_timeouts();
@@ -1168,7 +1182,7 @@ int flock_ntt_rs_encode_plan(flock_ctx* c, const uint64_t* msg, uint32_t log_msg
     size_t n = ((size_t)lanes) << log_msg_pos, nc = n << rate;
     DevBuf<f128> dm(n), dc(nc);
     CK(cudaMemcpyAsync(dm.p, msg, n * 16, cudaMemcpyHostToDevice, c->st));
-    ntt_rs_encode_plan(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, plan_index, c->st);
+    ntt_rs_encode_plan(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, plan_index, c->st, c->waits);
     CK(cudaMemcpyAsync(out, dc.p, nc * 16, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     check_device_timeouts();
@@ -1185,7 +1199,7 @@ int flock_ntt_autotune(flock_ctx* c, uint32_t log_msg_pos, uint32_t lanes, uint3
     double ms = -1;
     {
       DevBuf<f128> dc(((size_t)lanes) << log_d);
-      plan = ntt_autotune(dc.p, log_d, (int)lanes, (int)rate, c->st, &ms);
+      plan = ntt_autotune(dc.p, log_d, (int)lanes, (int)rate, c->st, c->waits, &ms);
     }
     if (best_ms) *best_ms = ms;
     if (desc && desc_cap) {
@@ -1306,9 +1320,11 @@ int flock_bench_ntt(flock_ctx* c, uint32_t log_msg_pos, uint32_t lanes, uint32_t
   return guard(c, [&] {
     size_t n = ((size_t)lanes) << log_msg_pos, nc = n << rate;
     DevBuf<f128> dm(n), dc(nc);
-    ntt_autotune(dc.p, (int)(log_msg_pos + rate), (int)lanes, (int)rate, c->st);
+    ntt_autotune(dc.p, (int)(log_msg_pos + rate), (int)lanes, (int)rate, c->st, c->waits);
     k_fill<<<(unsigned)((2 * n + 255) / 256), 256, 0, c->st>>>((uint64_t*)dm.p, 2 * n, 1);
-    *ms = time_launches(c->st, iters, [&] { ntt_rs_encode(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, c->st); });
+    *ms = time_launches(c->st, iters, [&] {
+      ntt_rs_encode(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, c->st, c->waits);
+    });
     return FLOCK_OK;
   });
 }
@@ -1337,7 +1353,7 @@ int flock_bench_ntt_plan(flock_ctx* c, uint32_t log_msg_pos, uint32_t lanes, uin
     DevBuf<f128> dm(n), dc(nc);
     k_fill<<<(unsigned)((2 * n + 255) / 256), 256, 0, c->st>>>((uint64_t*)dm.p, 2 * n, 1);
     *ms = time_launches(c->st, iters, [&] {
-      ntt_rs_encode_plan(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, plan_index, c->st);
+      ntt_rs_encode_plan(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, plan_index, c->st, c->waits);
     });
     return FLOCK_OK;
   });

@@ -185,6 +185,17 @@ struct DeviceTimeouts {
 };
 const DeviceTimeouts& device_timeouts();
 void check_device_timeouts();
+// What a launch's bounded waits take: the word they set when one ran out, and
+// after how many polls of an mbarrier one has (a poll suspends for up to 4 us, so
+// the default is a second, where microseconds are expected).  What the wait was
+// for is in flight still, so it is waited for kWaitPolls longer; the CTA then
+// starts nothing else, frees its tensor memory and returns.  With polls = 0
+// nothing is started at all, and the first wait runs out.
+constexpr unsigned kWaitPolls = 1u << 18;
+struct WaitLimit {
+  unsigned* ran_out = nullptr;
+  unsigned polls = kWaitPolls;
+};
 
 // K0
 void launch_witness_seed(uint64_t seed, uint32_t log2, uint32_t n_blocks, uint32_t n_slots, f128* z, f128* a,
@@ -237,7 +248,8 @@ using NttPlan = std::vector<NttPass>;
 // Times the candidate plans of a shape on `scratch` (lanes << log_d values,
 // overwritten), keeps the fastest for this device and returns it; later
 // encodes of the shape use it (untuned shapes use the default split).
-NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaStream_t s, double* best_ms = nullptr);
+NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaStream_t s, const WaitLimit& w,
+                     double* best_ms = nullptr);
 NttPlan ntt_plan(int log_d, int lanes, int layer_begin);
 const f128* ntt_evals(int log_d);  // device table of the per-layer basis values
 std::string ntt_plan_desc(const NttPlan& plan);
@@ -246,9 +258,10 @@ size_t ntt_plan_count(int log_d, int lanes, int layer_begin);
 // the description of candidate plan `index` ("" past the last one)
 std::string ntt_plan_desc_at(int log_d, int lanes, int layer_begin, size_t index);
 void ntt_rs_encode_plan(const f128* msg, f128* cw, int log_msg_pos, int lanes, int log_inv_rate, size_t plan_idx,
-                        cudaStream_t s);
-void ntt_rs_encode(const f128* msg, f128* cw, int log_msg_pos, int lanes, int log_inv_rate, cudaStream_t s);
-void ntt_forward(f128* data, int log_d, int lanes, int start_layer, cudaStream_t s);
+                        cudaStream_t s, const WaitLimit& w);
+void ntt_rs_encode(const f128* msg, f128* cw, int log_msg_pos, int lanes, int log_inv_rate, cudaStream_t s,
+                   const WaitLimit& w);
+void ntt_forward(f128* data, int log_d, int lanes, int start_layer, cudaStream_t s, const WaitLimit& w);
 void ntt_transposed_encode(f128* e, f128* out, int log_msg, int log_inv_rate, cudaStream_t s);
 // Fused multi-proof commit (serving / batching): one entry per proof of a
 // device-resident job table; every launch of the commit covers all jobs, a
@@ -282,7 +295,7 @@ void ntt_pass_batch(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_t
                     cudaStream_t s);
 // the jobs' kind-3 passes; max_R: the largest layer count among them
 void ntt_pass_batch_t(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_tiles, int max_R, int sms,
-                      cudaStream_t s);
+                      cudaStream_t s, const WaitLimit& w);
 void merkle_leaves_batch(const BatchJob* jobs, int n_jobs, uint64_t total, cudaStream_t s);
 void merkle_parents_batch(const BatchJob* jobs, int n_jobs, int level, uint64_t total, cudaStream_t s);
 void merkle_top_batch(const BatchJob* jobs, int n_jobs, cudaStream_t s);
@@ -335,7 +348,8 @@ void fold_pair_final(const f128* a_in, const f128* b_in, f128 rho, f128* out, cu
 // k: columns of the block matrices (2^k_log); comb: room for 2 k values
 void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_ptr, const uint16_t* bt_row,
              const f128* eq, f128 alpha, f128 beta, int pin, int k, f128* comb, cudaStream_t s);
-void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s);
+void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s,
+             const WaitLimit& w);
 void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s,
               const MailArgs& mail = {});
 // s_hat_v of the ab claim from the block-folded z (2^k_log values)

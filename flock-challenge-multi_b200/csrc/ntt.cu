@@ -288,21 +288,27 @@ constexpr int kSeqWords = 12;  // per twiddle: ten of its sequence, whether it i
 
 struct TmapCta {
   uint32_t tile, seqs, mat;  // shared addresses (mat: two matrices, 1024-byte aligned)
-  uint32_t bar, bar_ld;      // mbarriers of the products and of the tile's load
+  uint32_t bar;              // mbarriers of the products, of the tile's load, of the end; two words
   uint32_t taddr;            // tensor-memory base
   int warp;
   TmRows rows;
   uint32_t phase = 0, phase_ld = 0;
-  bool live = true;
-  __device__ __forceinline__ void wait(uint32_t b, uint32_t& ph) {
-    if (live) live = tm_wait(b, ph);
+  __device__ __forceinline__ uint32_t bar_ld() const { return bar + 8; }
+  __device__ __forceinline__ uint32_t bar_end() const { return bar + 16; }
+  // Set once a wait of the CTA ran out: from then on its threads run through
+  // their tiles without waiting, loading or starting products, on wrong values.
+  // In shared memory and read off the waits' path: with a flag per thread, tested
+  // between the barrier and the products' start, a pass takes 1.3 % longer.
+  __device__ __forceinline__ uint32_t dead() const { return bar + 28; }
+  __device__ __forceinline__ void wait(uint32_t b, uint32_t& ph, uint32_t polls) {
+    tm_wait(b, ph, dead(), polls);
     ph ^= 1;
   }
 };
 
 // Stage s of the tile in shared memory.
 template <bool LAST>
-__device__ __forceinline__ void ntt_stage_t(int R, int s, TmapCta& C, const TmShifts& sh) {
+__device__ __forceinline__ void ntt_stage_t(int R, int s, TmapCta& C, const TmShifts& sh, uint32_t polls) {
   const int tid = threadIdx.x, hb = LAST ? 0 : R - 1 - s;
   const uint32_t sq = C.seqs + 4 * kSeqWords * ((1 << s) - 1);
   const uint32_t my = C.taddr + ((uint32_t)(tid & ~31) << 16);  // this warp's 32 lanes
@@ -329,12 +335,13 @@ __device__ __forceinline__ void ntt_stage_t(int R, int s, TmapCta& C, const TmSh
       tm_fence_smem();
       cur = k;
     }
+    const uint32_t dead = tm_lds32(C.dead());
     tm_put_wait();
     tm_fence_before();
     __syncthreads();
     if (C.warp == 0) {
       tm_fence_after();
-      if (tm_elect()) {
+      if (tm_elect() && !dead) {
         const uint64_t desc = tm_desc(C.mat);
         if (LAST) {
           tm_mma(C.taddr, C.taddr + kTmOperand, desc, 0, ~0u);
@@ -352,7 +359,7 @@ __device__ __forceinline__ void ntt_stage_t(int R, int s, TmapCta& C, const TmSh
   // passes behind the extraction.
   if (u < n_units) start(u);
   for (; u < n_units; u++) {
-    C.wait(C.bar, C.phase);
+    C.wait(C.bar, C.phase, polls);
     tm_fence_after();
     uint32_t r[32];
     tm_get(my, r);
@@ -370,7 +377,7 @@ __device__ __forceinline__ void ntt_stage_t(int R, int s, TmapCta& C, const TmSh
 // shared memory (~0: none); tiles of one prefix are neighbours, so a CTA that
 // runs successive tiles derives them rarely, except in the last pass.
 __device__ __forceinline__ void ntt_tile_t(const PassArgs& p, uint64_t t_id, uint32_t* seqs, TmapCta& C,
-                                           uint64_t& seq_hi, const TmShifts& sh) {
+                                           uint64_t& seq_hi, const TmShifts& sh, uint32_t polls) {
   const int R = p.R;
   const int log_d = p.log_d, l0 = p.l0;
   const int lo_bits = log_d - l0 - R;
@@ -384,9 +391,12 @@ __device__ __forceinline__ void ntt_tile_t(const PassArgs& p, uint64_t t_id, uin
   f128* const dst = p.data + ((hi << (log_d - l0)) | lo) * p.lanes + row;
   if (C.warp == 0) {  // a row of 64 values per lane (R <= 5)
     tm_store_read();  // the previous tile has left shared memory
-    if (tid == 0) tm_expect(C.bar_ld, 1024u << R);
+    // (no wait lies between the last tile's end and here: one value for the warp)
+    const bool live = __all_sync(0xffffffffu, polls && !tm_lds32(C.dead()));
+    if (tid == 0 && live) tm_expect(C.bar_ld(), 1024u << R);
     __syncwarp();
-    if (tid < (1 << R)) tm_load_row(C.tile + 1024 * tid, p.src ? p.src + lo * p.lanes + row : dst, 1024, C.bar_ld);
+    if (tid < (1 << R) && live)
+      tm_load_row(C.tile + 1024 * tid, p.src ? p.src + lo * p.lanes + row : dst, 1024, C.bar_ld());
   }
   if (hi != seq_hi) {
     for (int k = tid; k < (1 << R) - 1; k += 128) {
@@ -406,9 +416,9 @@ __device__ __forceinline__ void ntt_tile_t(const PassArgs& p, uint64_t t_id, uin
     seq_hi = hi;
     __syncthreads();
   }
-  C.wait(C.bar_ld, C.phase_ld);
-  for (int s = 0; s < R - 1; s++) ntt_stage_t<false>(R, s, C, sh);
-  ntt_stage_t<true>(R, R - 1, C, sh);
+  C.wait(C.bar_ld(), C.phase_ld, polls);
+  for (int s = 0; s < R - 1; s++) ntt_stage_t<false>(R, s, C, sh, polls);
+  ntt_stage_t<true>(R, R - 1, C, sh, polls);
   if (tid < (1 << R)) {
     tm_store_row(dst, C.tile + 1024 * tid, 1024);
     tm_store_commit();
@@ -425,12 +435,12 @@ struct TmapSetup {
     uint8_t* tile = mat + 2 * kTmMatBytes;
     seqs = reinterpret_cast<uint32_t*>(tile + ((size_t)1024 << R));
     uint64_t* bar = reinterpret_cast<uint64_t*>(seqs + ((size_t)kSeqWords << R));
-    uint32_t* slot = reinterpret_cast<uint32_t*>(bar + 2);
+    uint32_t* slot = reinterpret_cast<uint32_t*>(bar + 3);  // [tensor-memory address, dead]
     cta.warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     if (cta.warp == 0) tm_alloc(slot);
     if (threadIdx.x == 0) {
-      tm_mbar_init(bar);
-      tm_mbar_init(bar + 1);
+      for (int i = 0; i < 3; i++) tm_mbar_init(bar + i);
+      slot[1] = 0;
     }
     tm_fence_before();
     __syncthreads();
@@ -439,12 +449,15 @@ struct TmapSetup {
     cta.seqs = tm_smem(seqs);
     cta.mat = tm_smem(mat);
     cta.bar = tm_smem(bar);
-    cta.bar_ld = tm_smem(bar + 1);
     cta.taddr = __shfl_sync(0xffffffffu, *slot, 0);
     cta.rows = tm_rows(cta.mat);
   }
-  __device__ __forceinline__ void finish(unsigned* timeouts) {
-    if (!cta.live && threadIdx.x == 0) *timeouts = 1;
+  __device__ __forceinline__ void finish(const WaitLimit& w) {
+    if (tm_lds32(cta.dead())) {  // (set before the last tile's last barrier, if at all)
+      // products that were started before the thread that starts them saw the word
+      if (cta.warp == 0 && tm_elect()) tm_drain(cta.bar_end());
+      if (threadIdx.x == 0) *w.ran_out = 1;
+    }
     tm_store_done();
     tm_fence_before();
     __syncthreads();
@@ -454,13 +467,13 @@ struct TmapSetup {
 
 // per: successive tiles of a CTA
 __global__ void __launch_bounds__(128, 4) k_ntt_pass_t(PassArgs p, uint64_t n_tiles, uint64_t per, TmShifts sh,
-                                                       unsigned* __restrict__ timeouts) {
+                                                       WaitLimit w) {
   extern __shared__ __align__(16) uint8_t raw[];
   TmapSetup S(raw, p.R);
   uint64_t seq_hi = ~0ull;
   const uint64_t t0 = blockIdx.x * per, t1 = min(t0 + per, n_tiles);
-  for (uint64_t t = t0; t < t1; t++) ntt_tile_t(p, t, S.seqs, S.cta, seq_hi, sh);
-  S.finish(timeouts);
+  for (uint64_t t = t0; t < t1; t++) ntt_tile_t(p, t, S.seqs, S.cta, seq_hi, sh, w.polls);
+  S.finish(w);
 }
 
 template <bool TRANSPOSE, int KIND>
@@ -504,7 +517,7 @@ __global__ void __launch_bounds__(256, 2) k_ntt_pass_batch(const BatchJob* __res
 // The same for the jobs whose pass runs on the tensor cores.
 __global__ void __launch_bounds__(128, 4) k_ntt_pass_batch_t(const BatchJob* __restrict__ jobs, int n_jobs, int pass,
                                                              uint64_t total_tiles, uint64_t per, int max_R, TmShifts sh,
-                                                             unsigned* __restrict__ timeouts) {
+                                                             WaitLimit w) {
   extern __shared__ __align__(16) uint8_t raw[];
   TmapSetup S(raw, max_R);
   uint64_t seq_hi = ~0ull;
@@ -526,9 +539,9 @@ __global__ void __launch_bounds__(128, 4) k_ntt_pass_batch_t(const BatchJob* __r
     }
     if (lo != job) seq_hi = ~0ull;
     job = lo;
-    ntt_tile_t(a, t - J.tile0t[pass], S.seqs, S.cta, seq_hi, sh);
+    ntt_tile_t(a, t - J.tile0t[pass], S.seqs, S.cta, seq_hi, sh, w.polls);
   }
-  S.finish(timeouts);
+  S.finish(w);
 }
 
 __global__ void k_replicate_batch(const BatchJob* __restrict__ jobs, int n_jobs, uint64_t total) {
@@ -806,7 +819,7 @@ void launch_pass_w(const NttPass& ps, const PassArgs& a, uint64_t tiles, cudaStr
 }
 
 void launch_pass(const NttPass& ps, f128* data, const f128* ev, int log_d, int lanes, bool transpose,
-                 cudaStream_t s, const f128* src = nullptr) {
+                 cudaStream_t s, const WaitLimit& w, const f128* src = nullptr) {
   PassArgs a{data, ev, log_d, lanes, ps.lgs, ps.l0, ps.R};
   if (src) {
     a.src = src;
@@ -816,11 +829,11 @@ void launch_pass(const NttPass& ps, f128* data, const f128* ev, int log_d, int l
   const uint64_t tiles = ((uint64_t)1 << (log_d - ps.R)) * (uint64_t)(lanes >> ps.lgs);
   if (ps.kind == 3) {
     if (transpose) throw CudaError("ntt: tensor passes run forward only");
+    if (!w.ran_out) throw CudaError("ntt: a tensor pass needs a word for its waits");
     CK(cudaFuncSetAttribute(k_ntt_pass_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_t_smem(kMaxRt)));
     const uint64_t per = tiles_per_cta(tiles, 148);
     count_launch();
-    k_ntt_pass_t<<<(unsigned)((tiles + per - 1) / per), 128, pass_t_smem(ps.R), s>>>(a, tiles, per, tm_shifts(),
-                                                                                    device_timeouts().dev);
+    k_ntt_pass_t<<<(unsigned)((tiles + per - 1) / per), 128, pass_t_smem(ps.R), s>>>(a, tiles, per, tm_shifts(), w);
     return;
   }
   if (ps.kind) {
@@ -919,17 +932,19 @@ NttPlan plan_for(int log_d, int lanes, int layer_begin) {
 // src != nullptr (forward only): the message whose replicate the first pass
 // reads in place of data
 void run_plan(const NttPlan& plan, f128* data, int log_d, int lanes, bool transpose, cudaStream_t s,
-              const f128* src = nullptr) {
+              const WaitLimit& w, const f128* src = nullptr) {
   if (plan.empty()) return;
   const f128* ev = device_evals(log_d);
   if (transpose)
-    for (auto it = plan.rbegin(); it != plan.rend(); ++it) launch_pass(*it, data, ev, log_d, lanes, true, s);
+    for (auto it = plan.rbegin(); it != plan.rend(); ++it) launch_pass(*it, data, ev, log_d, lanes, true, s, w);
   else
-    for (size_t i = 0; i < plan.size(); i++) launch_pass(plan[i], data, ev, log_d, lanes, false, s, i ? nullptr : src);
+    for (size_t i = 0; i < plan.size(); i++)
+      launch_pass(plan[i], data, ev, log_d, lanes, false, s, w, i ? nullptr : src);
 }
 
-void run_passes(f128* data, int log_d, int lanes, int layer_begin, bool transpose, cudaStream_t s) {
-  run_plan(plan_for(log_d, lanes, layer_begin), data, log_d, lanes, transpose, s);
+void run_passes(f128* data, int log_d, int lanes, int layer_begin, bool transpose, cudaStream_t s,
+                const WaitLimit& w) {
+  run_plan(plan_for(log_d, lanes, layer_begin), data, log_d, lanes, transpose, s, w);
 }
 }  // namespace
 
@@ -949,16 +964,17 @@ void ntt_pass_batch(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_t
 }
 
 void ntt_pass_batch_t(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_tiles, int max_R, int sms,
-                      cudaStream_t s) {
+                      cudaStream_t s, const WaitLimit& w) {
   const size_t smem = pass_t_smem(max_R);
   CK(cudaFuncSetAttribute(k_ntt_pass_batch_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_t_smem(kMaxRt)));
   const uint64_t per = tiles_per_cta(total_tiles, sms);
   count_launch();
   k_ntt_pass_batch_t<<<(unsigned)((total_tiles + per - 1) / per), 128, smem, s>>>(
-      jobs, n_jobs, pass, total_tiles, per, max_R, tm_shifts(), device_timeouts().dev);
+      jobs, n_jobs, pass, total_tiles, per, max_R, tm_shifts(), w);
 }
 
-NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaStream_t s, double* best_ms) {
+NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaStream_t s, const WaitLimit& w,
+                     double* best_ms) {
   int dev = 0;
   CK(cudaGetDevice(&dev));
   const PlanKey key{dev, log_d, lanes, layer_begin};
@@ -985,11 +1001,11 @@ NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaS
   // one warm launch, then the best of two timed launches (CUDA events on
   // the launching stream), on the random scratch filled above
   auto time_pass = [&](const NttPass& ps) {
-    launch_pass(ps, scratch, ev, log_d, lanes, false, s);
+    launch_pass(ps, scratch, ev, log_d, lanes, false, s, w);
     float best = 1e30f;
     for (int r = 0; r < 2; r++) {
       CK(cudaEventRecord(e0, s));
-      launch_pass(ps, scratch, ev, log_d, lanes, false, s);
+      launch_pass(ps, scratch, ev, log_d, lanes, false, s, w);
       CK(cudaEventRecord(e1, s));
       CK(cudaEventSynchronize(e1));
       float t = 0;
@@ -1067,20 +1083,21 @@ std::string ntt_plan_desc_at(int log_d, int lanes, int layer_begin, size_t index
 }
 
 void ntt_rs_encode_plan(const f128* msg, f128* cw, int log_msg_pos, int lanes, int log_inv_rate, size_t plan_idx,
-                        cudaStream_t s) {
+                        cudaStream_t s, const WaitLimit& w) {
   const int log_d = log_msg_pos + log_inv_rate;
   auto plans = all_plans(log_d, lanes, log_inv_rate);
   if (plan_idx >= plans.size()) throw std::out_of_range("ntt plan index");
   size_t msg_len = ((size_t)lanes) << log_msg_pos;
   if (plans[plan_idx].empty() || plans[plan_idx][0].l0 != log_inv_rate) {
     count_launch(); k_replicate<<<(unsigned)((msg_len + 255) / 256), 256, 0, s>>>(msg, cw, msg_len, 1 << log_inv_rate);
-    run_plan(plans[plan_idx], cw, log_d, lanes, false, s);
+    run_plan(plans[plan_idx], cw, log_d, lanes, false, s, w);
   } else {
-    run_plan(plans[plan_idx], cw, log_d, lanes, false, s, msg);
+    run_plan(plans[plan_idx], cw, log_d, lanes, false, s, w, msg);
   }
 }
 
-void ntt_rs_encode(const f128* msg, f128* cw, int log_msg_pos, int lanes, int log_inv_rate, cudaStream_t s) {
+void ntt_rs_encode(const f128* msg, f128* cw, int log_msg_pos, int lanes, int log_inv_rate, cudaStream_t s,
+                   const WaitLimit& w) {
   const int log_d = log_msg_pos + log_inv_rate;
   const NttPlan plan = plan_for(log_d, lanes, log_inv_rate);
   if (plan.empty()) {  // no butterfly layer: the codeword is the replicate
@@ -1088,17 +1105,17 @@ void ntt_rs_encode(const f128* msg, f128* cw, int log_msg_pos, int lanes, int lo
     count_launch(); k_replicate<<<(unsigned)((msg_len + 255) / 256), 256, 0, s>>>(msg, cw, msg_len, 1 << log_inv_rate);
     return;
   }
-  run_plan(plan, cw, log_d, lanes, false, s, msg);  // the first pass reads the message's replicate in place
+  run_plan(plan, cw, log_d, lanes, false, s, w, msg);  // the first pass reads the message's replicate in place
 }
 
-void ntt_forward(f128* data, int log_d, int lanes, int start_layer, cudaStream_t s) {
-  run_passes(data, log_d, lanes, start_layer, false, s);
+void ntt_forward(f128* data, int log_d, int lanes, int start_layer, cudaStream_t s, const WaitLimit& w) {
+  run_passes(data, log_d, lanes, start_layer, false, s, w);
 }
 
 // out[j] (j < 2^log_msg) = sum_q E[q] * (codeword position q of unit message j);
 // e is overwritten.
 void ntt_transposed_encode(f128* e, f128* out, int log_msg, int log_inv_rate, cudaStream_t s) {
-  run_passes(e, log_msg + log_inv_rate, 1, log_inv_rate, true, s);
+  run_passes(e, log_msg + log_inv_rate, 1, log_inv_rate, true, s, WaitLimit{});  // (no kernel of these waits)
   size_t len = (size_t)1 << log_msg;
   count_launch(); k_fold_copies<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(e, out, len, 1 << log_inv_rate);
 }

@@ -124,6 +124,7 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   mail_block = pinned_take(kMailBytes);
   d_ticket = dalloc<unsigned>(1, st);
   mail = mailbox_at(mail_block, d_ticket);
+  waits.ran_out = device_timeouts().dev;
   h_out = static_cast<f128*>(pinned_take(1024 * sizeof(f128)));
   h_stage = static_cast<uint8_t*>(pinned_take(kStageBytes));
   const Statement& S = statement(hash);
@@ -157,13 +158,13 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
 // 1/2), each Ligero level, and the transposed encodes of the query-basis
 // induction (one lane).
 void Setup::tune_ntt_plans() {
-  ntt_autotune(cw0, m - 12, 64, 1, st);
-  for (auto& L : levels) ntt_autotune(L.cw, L.log_msg_pos + L.rate, L.lanes, L.rate, st);
+  ntt_autotune(cw0, m - 12, 64, 1, st, waits);
+  for (auto& L : levels) ntt_autotune(L.cw, L.log_msg_pos + L.rate, L.lanes, L.rate, st, waits);
   int n = m - 7 - lad->initial_k;
-  ntt_autotune(induce_buf, n + lad->rate[0], 1, lad->rate[0], st);
+  ntt_autotune(induce_buf, n + lad->rate[0], 1, lad->rate[0], st, waits);
   for (size_t i = 0; i + 1 < lad->ks.size(); i++) {
     n -= lad->ks[i];
-    ntt_autotune(induce_buf, n + levels[i].rate, 1, levels[i].rate, st);
+    ntt_autotune(induce_buf, n + levels[i].rate, 1, levels[i].rate, st, waits);
   }
   CK(cudaStreamSynchronize(st));
 }
@@ -202,7 +203,7 @@ cudaGraphExec_t capture(cudaStream_t st, uint64_t* launches, F&& body) {
 void Setup::capture_commit() {
   const char* env = getenv("FLOCK_COMMIT_GRAPHS");
   if (env && strcmp(env, "0") == 0) return;
-  commit_graph[0] = capture(st, &commit_launches[0], [&] { ntt_rs_encode(z, cw0, m - 13, 64, 1, st); });
+  commit_graph[0] = capture(st, &commit_launches[0], [&] { ntt_rs_encode(z, cw0, m - 13, 64, 1, st, waits); });
   commit_graph[1] =
       capture(st, &commit_launches[1], [&] { merkle_build(cw0, n_leaves0, 64 * 16, tree0, merkle_fn, st); });
 }
@@ -293,7 +294,7 @@ BatchCommit batch_commit_async(const std::vector<Setup*>& setups, const std::vec
       // pass 0 reads each job's message as its replicated codeword
       for (int p = 0; p < max_pass; p++) {
         if (tiles[p]) ntt_pass_batch(dj, n, p, tiles[p], smem, 2 * sms, st);
-        if (tiles_t[p]) ntt_pass_batch_t(dj, n, p, tiles_t[p], max_R, sms, st);
+        if (tiles_t[p]) ntt_pass_batch_t(dj, n, p, tiles_t[p], max_R, sms, st, setups[0]->waits);
       }
       merkle_leaves_batch(dj, n, leaves, st);
       for (int l = 1; l <= max_level; l++) merkle_parents_batch(dj, n, l, par[l], st);
@@ -509,7 +510,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
       CK(cudaGraphLaunch(commit_graph[0], st));
       count_launch(commit_launches[0]);
     } else {
-      ntt_rs_encode(z, cw0, m - 13, 64, 1, st);
+      ntt_rs_encode(z, cw0, m - 13, 64, 1, st, waits);
     }
   }
   mark(2);
@@ -774,7 +775,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     else lc_comb(at_ptr, at_row, bt_ptr, bt_row, eq_inner, alpha, beta, statement(hash).z_const, kk, comb, st);
     eq_table(x_outer, scratch_eq());
     CK(cudaMemsetAsync(zv, 0, kk * sizeof(f128), st));
-    lc_zvec(z, scratch_eq(), (size_t)1 << (m - k_log), k_log, zv, gs, st);
+    lc_zvec(z, scratch_eq(), (size_t)1 << (m - k_log), k_log, zv, gs, st, waits);
     // pre-sumcheck z_vec: the ab-claim's ring-switch statistic is read from it
     CK(cudaMemcpyAsync(zv_pre, zv, kk * sizeof(f128), cudaMemcpyDeviceToDevice, st));
   }
@@ -1125,7 +1126,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   mark(8);
   // level 1 commit
   auto commit = [&](Level& L) {
-    ntt_rs_encode(f, L.cw, L.log_msg_pos, L.lanes, L.rate, st);
+    ntt_rs_encode(f, L.cw, L.log_msg_pos, L.lanes, L.rate, st, waits);
     H32 rt;
     if (merkle_fn != kFnSha256 && L.positions > 1) {  // the tree's last kernel posts the root
       merkle_build(L.cw, L.positions, (size_t)L.lanes * 16, L.tree, st, mail.next(2));

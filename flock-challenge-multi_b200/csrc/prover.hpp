@@ -153,6 +153,9 @@ class Setup {
   // the Fiat-Shamir transcript's hash (FsChallenger::with_hash); settable
   // between proofs
   int fs_fn = kFnBlake3;
+  // the bounded waits of this setup's kernels (the captured commit keeps those
+  // of its construction); polls settable between proofs
+  WaitLimit waits;
   int n_log = 0, m = 0, sms = 0;
   // SMs the grid-stride kernels of this setup spread over (0: all).  The
   // serving queue lowers it for large proofs so that their long persistent

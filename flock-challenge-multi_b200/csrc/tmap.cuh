@@ -7,7 +7,8 @@
 // is a byte matrix in shared memory (B operand), and a result bit is the
 // parity of a 32-bit count.  Two result bits share one count: the matrix
 // byte is m_n + 128 m_n', so bit 0 of the count is the parity of bit n and
-// bit 7 that of bit n' (the first count is at most 127: see tm_safe below).
+// bit 7 that of bit n' (the first count is at most 127 unless a row of the
+// matrix is all ones: tensor_safe, ntt.cu, checks the twiddles).
 // N is therefore 64, not 128, which halves both the tensor work and the
 // extraction, the part that runs on the integer pipe.
 //
@@ -27,14 +28,11 @@
 // GHASH reduction of an overflow makes).  So a matrix is written from 32
 // bytes of Q by funnel shifts, with no field arithmetic.
 #pragma once
-#include "gf128.cuh"
+#include "kernels.cuh"
 
 constexpr int kTmMatBytes = 8192;    // one matrix: 64 rows of 128 bytes, 128-byte swizzle
 constexpr int kTmCols = 128;         // tensor-memory columns of one CTA: result 64, operand 32 (x 2)
 constexpr uint32_t kTmOperand = 64;  // first operand column
-// tries of an mbarrier wait before it is given up (each try suspends for up
-// to a hardware time slice; a product takes under a microsecond)
-constexpr int kTmWaitTries = 1 << 20;
 
 __device__ __forceinline__ uint32_t tm_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -50,6 +48,9 @@ __device__ __forceinline__ uint32_t tm_lds32(uint32_t a) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
   return v;
+}
+__device__ __forceinline__ void tm_sts32(uint32_t a, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 // predicated, without a branch; OFF: bytes added to the address
 template <int OFF>
@@ -93,19 +94,29 @@ __device__ __forceinline__ void tm_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tm_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tm_fence_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// Waits for phase `parity`; false when it did not come within the limit.
-__device__ __forceinline__ bool tm_wait(uint32_t a, uint32_t parity) {
-  for (int i = 0; i < kTmWaitTries; i++) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
+__device__ __forceinline__ bool tm_poll(uint32_t a, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(a), "r"(parity)
+      : "memory");
+  return ok;
+}
+// Waits for phase `parity`.  When it has not come within `polls` polls, what was
+// in flight is waited for kWaitPolls longer, and then the CTA's word `dead` (a
+// shared address) is set: false, here and at once in every later wait that finds
+// its phase not come.  The CTA starts nothing from then on.
+__device__ __forceinline__ bool tm_wait(uint32_t a, uint32_t parity, uint32_t dead, uint32_t polls) {
+  if (tm_poll(a, parity)) return true;
+  if (tm_lds32(dead)) return false;
+  for (uint32_t i = 0; i < polls; i++)
+    if (tm_poll(a, parity)) return true;
+  for (uint32_t i = 0; i < kWaitPolls; i++)
+    if (tm_poll(a, parity)) break;
+  tm_sts32(dead, 1);
   return false;
 }
 
@@ -136,6 +147,14 @@ __device__ __forceinline__ void tm_mma(uint32_t d, uint32_t a, uint64_t desc) {
 __device__ __forceinline__ void tm_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
+}
+
+// The thread that started products waits for all of them, on an mbarrier not used
+// before (bounded; the end of a CTA that gave up).
+__device__ __forceinline__ void tm_drain(uint32_t bar) {
+  tm_commit(bar);
+  for (uint32_t i = 0; i < kWaitPolls && !tm_poll(bar, 0); i++) {
+  }
 }
 
 // Powers of two that reach the kernels as parameters: a product by one is an

@@ -60,12 +60,12 @@ __device__ __forceinline__ void gemm_mma(uint32_t d, uint64_t a, uint64_t b, boo
 __device__ __forceinline__ void copy4(uint32_t dst, const void* src, bool there) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(there ? 4 : 0) : "memory");
 }
-__global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, unsigned* __restrict__ timeouts) {
+__global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, WaitLimit W) {
   extern __shared__ __align__(16) uint8_t raw[];
   const uint32_t base = tm_smem(raw) + ((1024 - (tm_smem(raw) & 1023)) & 1023);
   const uint32_t slots = base + kBufs * kBufBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(raw + (slots - tm_smem(raw)) + kAhead * kSpreaders * kSlotBytes);
-  uint32_t* addr = reinterpret_cast<uint32_t*>(bars + kBufs);
+  uint32_t* addr = reinterpret_cast<uint32_t*>(bars + kBufs + 1);  // [tensor-memory address, dead, taken]
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tm_smem(addr)),
@@ -73,29 +73,32 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, unsigne
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (tid == 0)
-    for (int i = 0; i < kBufs; i++) tm_mbar_init(bars + i);
+  if (tid == 0) {
+    for (int i = 0; i < kBufs + 1; i++) tm_mbar_init(bars + i);  // a buffer's products are done; all are
+    addr[1] = addr[2] = 0;
+  }
   tm_fence_before();
   __syncthreads();
   tm_fence_after();
   const uint32_t taddr = __shfl_sync(0xffffffffu, *addr, 0), bar = tm_smem(bars);
+  const uint32_t dead = tm_smem(addr + 1), taken = tm_smem(addr + 2);
 
   const uint32_t per_col = (G.n_rows + kRowsStep - 1) / kRowsStep;
   const uint64_t total = (uint64_t)per_col * G.cols;
   const uint32_t s0 = (uint32_t)(total * blockIdx.x / gridDim.x), s1 = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x);
   const uint32_t steps = s1 - s0;
-  bool live = true;
   // step n: buffer n mod kBufs, use n / kBufs of it; column and row block of step s0 + n
   uint32_t col = s0 / per_col, blk = s0 % per_col;
 
   if (warp == kSpreaders / 32) {
     for (uint32_t n = 0, buf = 0; n < steps; n++) {
+      const bool go = W.polls && !tm_lds32(dead);
       // named barrier 1 + buf: the step's operands are in place
       asm volatile("bar.sync %0, %1;" ::"r"(1 + buf), "n"(kGemmThreads) : "memory");
       tm_fence_after();
       const uint32_t A = base + buf * kBufBytes, B = A + 2 * kTileBytes;
       const bool first = n == 0 || blk == 0;
-      if (tm_elect()) {
+      if (tm_elect() && go) {
 #pragma unroll
         for (int k = 0; k < 2; k++)  // 32 rows an instruction
 #pragma unroll
@@ -103,10 +106,14 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, unsigne
             gemm_mma(taddr + 128 * t, tm_desc(A + t * kTileBytes + 4096 * k), tm_desc(B + 4096 * k), !first || k);
         tm_commit(bar + 8 * buf);
       }
+      if (lane == 0) tm_sts32(taken, n + 1);
       __syncwarp();
       buf = buf + 1 == kBufs ? 0 : buf + 1;
       if (++blk == per_col) blk = 0;
     }
+    // whoever gave up, the products end before their memory is another CTA's
+    if (tm_elect()) tm_drain(bar + 8 * kBufs);
+    __syncwarp();
   } else {
     const int r0 = tid >> 3, bw = tid & 7;  // two words of bits (rows r0, r0 + 32), one of a weight (row tid / 4)
     const uint32_t slot = slots + tid * kSlotBytes;
@@ -130,6 +137,11 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, unsigne
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // No wait of this thread ran out, nor did it see another's.  If one did, it
+    // goes on to the end with wrong values, and before it arrives waits, in place
+    // of the products, for the ninth warp to have taken the barrier's last round:
+    // that warp waits for nothing but these arrivals.
+    bool live = true;
     for (int i = 0; i < kAhead - 1; i++) fetch(i);
     for (uint32_t n = 0, buf = 0, use = 0; n < steps; n++) {
       fetch(n + kAhead - 1);
@@ -137,7 +149,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, unsigne
       const uint32_t d = slot + (n % kAhead) * (kSpreaders * kSlotBytes);
       const uint32_t x[2] = {tm_lds32(d), tm_lds32(d + 4)}, w = tm_lds32(d + 8);
       const uint32_t A = base + buf * kBufBytes, B = A + 2 * kTileBytes;
-      if (use && live) live = tm_wait(bar + 8 * buf, (use - 1) & 1);  // the buffer's last products have read it
+      if (use && live) live = tm_wait(bar + 8 * buf, (use - 1) & 1, dead, W.polls);  // its last products have read it
+      if (use && !live)
+        for (uint32_t i = 0; i < kWaitPolls && tm_lds32(taken) + kBufs <= n; i++) __nanosleep(20);
       uint4 lo, hi;
 #pragma unroll
       for (int i = 0; i < 2; i++) {
@@ -156,9 +170,11 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, unsigne
       }
       tm_fence_smem();
       tm_fence_before();  // (a finished column's counts have been read)
+      __syncwarp();
       asm volatile("bar.arrive %0, %1;" ::"r"(1 + buf), "n"(kGemmThreads) : "memory");
       if (n + 1 == steps || blk + 1 == per_col) {  // the column's or this CTA's last rows: extract
-        if (live) live = tm_wait(bar + 8 * buf, use & 1);
+        if (live) live = tm_wait(bar + 8 * buf, use & 1, dead, W.polls);
+        __syncwarp();
         tm_fence_after();
         // warps 0..3 read the first tile, 4..7 the second: row 32 (warp mod 4) + lane
         const uint32_t src = taddr + ((uint32_t)(warp & 3) << 21) + 128 * (warp >> 2);
@@ -184,9 +200,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, unsigne
       }
     }
   }
-  if (!live) *timeouts = 1;
   tm_fence_before();
   __syncthreads();
+  if (tid == 0 && tm_lds32(dead)) *W.ran_out = 1;
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(kGemmCols) : "memory");
 }
@@ -195,7 +211,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, unsigne
 
 // zv[i] ^= XOR over o < n_outer with bit i of o's 2^k_log-bit block set of eqo[o]
 // (sms: the SMs the launch may fill, one wave of resident CTAs on them)
-void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s) {
+void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s,
+             const WaitLimit& w) {
+  if (!w.ran_out) throw CudaError("lc_zvec: a word for its waits");
   if (k_log < 8 || k_log > 17 || n_outer >> 30) throw CudaError("lc_zvec: bad shape");
   GemmArgs G{reinterpret_cast<const uint32_t*>(z), 1u << (k_log - 5), (uint32_t)n_outer, 1u << (k_log - 8),
              reinterpret_cast<const uint32_t*>(eqo), zv};
@@ -204,5 +222,5 @@ void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv
   const uint64_t grid = (uint64_t)resident_grid((const void*)k_lc_zvec, kGemmThreads, kGemmSmem, sms);
   count_launch();
   k_lc_zvec<<<(unsigned)std::max<uint64_t>(1, std::min(grid, steps)), kGemmThreads, kGemmSmem, s>>>(
-      G, device_timeouts().dev);
+      G, w);
 }

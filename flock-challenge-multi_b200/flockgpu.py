@@ -44,6 +44,7 @@ EXPORTS = (
     "flock_zerocheck_round1_deg4", "flock_bench_round1_deg4", "flock_keccak3_setup_create",
     "flock_keccak3_verify_bundle", "flock_keccak3_statement_digest", "flock_keccak3_witness", "flock_keccak3_comb",
     "flock_sha256_prove_chain", "flock_sha256_chain_blocks", "flock_keccak_prove_chain", "flock_keccak_chain_states",
+    "flock_setup_set_wait_polls", "flock_ctx_set_wait_polls",
 )
 # the hash behind Merkle trees / the transcript (HashKind discriminants)
 HASH = {"sha256": 0, "blake3": 1}
@@ -125,6 +126,8 @@ def load() -> ctypes.CDLL:
         lib.flock_bench_prove.argtypes = [vp, u64, i32, ctypes.POINTER(ctypes.c_double), vp,
                                           ctypes.POINTER(u64)]
         lib.flock_merkle_root_noalloc.argtypes = [vp, sz, sz, vp, vp]
+        lib.flock_setup_set_wait_polls.argtypes = [vp, u32]
+        lib.flock_ctx_set_wait_polls.argtypes = [vp, u32]
         lib.flock_serve_start.argtypes = [vp, i32]
         lib.flock_serve_prewarm.argtypes = [vp, u32, i32, ctypes.POINTER(i32)]
         lib.flock_zerocheck_round1_deg4.argtypes = [vp, vp, vp, vp, vp, vp, u32, vp, vp, vp]
@@ -401,6 +404,10 @@ class Context:
             self.close()
         except Exception:
             pass
+
+    def set_wait_polls(self, polls: int) -> None:
+        """The limit of the bounded waits of the kernels that this context's own calls launch."""
+        self._check(self.lib.flock_ctx_set_wait_polls(self.h, polls), "ctx_set_wait_polls")
 
     # ---- serving (continuous batching of proof jobs) ----
     def serve_start(self, slots: int = 4) -> None:
@@ -961,6 +968,10 @@ class Prover:
             self.close()
         except Exception:
             pass
+
+    def set_wait_polls(self, polls: int) -> None:
+        """The limit of the bounded waits of the kernels of this setup's proofs."""
+        self.ctx._check(self.ctx.lib.flock_setup_set_wait_polls(self.h, polls), "setup_set_wait_polls")
 
     def prove_seed(self, seed: int, domain: bytes = DOMAIN) -> bytes:
         n = ctypes.c_size_t()

@@ -124,6 +124,14 @@ int flock_setup_set_transcript(flock_setup* s, int hash);
 /* The transcript hash of the context's verify-bundle entry points (the
  * bundle records its Merkle hash but not its transcript's). */
 int flock_ctx_set_transcript(flock_ctx* ctx, int hash);
+/* After how many polls (of up to 4 us each) a kernel gives up a wait for its own
+ * copies or tensor-core products; the call that launched it then returns
+ * FLOCK_ERR_CUDA.  Default 2^18, a second where microseconds are expected.  With 0 the kernels start nothing that they wait for, so that each
+ * first wait runs out (how the error path is tested).  Of a setup's proofs (their
+ * captured commitment keeps the default) / of the context's own calls.  Not while
+ * one of them runs. */
+int flock_setup_set_wait_polls(flock_setup* s, uint32_t polls);
+int flock_ctx_set_wait_polls(flock_ctx* ctx, uint32_t polls);
 
 /* One proof; inputs generated on the GPU from `seed` exactly as the
  * benchmark generator does.  Writes the FLOCK v4 bundle bytes. */
