@@ -53,18 +53,11 @@ std::atomic<uint64_t>& kernel_launch_counter() {
   return n;
 }
 
-const DeviceTimeouts& device_timeouts() {
-  static const DeviceTimeouts d = [] {
-    void *h = nullptr, *g = nullptr;
-    CK(cudaHostAlloc(&h, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable));
-    *static_cast<unsigned*>(h) = 0;
-    CK(cudaHostGetDevicePointer(&g, h, 0));
-    return DeviceTimeouts{static_cast<unsigned*>(h), static_cast<unsigned*>(g)};
-  }();
-  return d;
-}
-void check_device_timeouts() {
-  if (*device_timeouts().host) throw CudaError("a kernel's bounded wait ran out");
+void check_waits(const WaitLimit& w) {
+  volatile unsigned* word = w.ran_out;
+  if (!word || !*word) return;
+  *word = 0;
+  throw CudaError("a kernel's bounded wait ran out");
 }
 
 int resident_grid(const void* kernel, int threads, size_t smem, int sms) {
@@ -164,11 +157,13 @@ int flock_ctx_create(int device, uint64_t hbm_budget_bytes, flock_ctx** out) {
     CK(cudaSetDevice(device));
     CK(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device));
     CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
-    c->waits.ran_out = device_timeouts().dev;
+    c->waits.ran_out = static_cast<unsigned*>(flock::pinned_take(sizeof(unsigned)));
+    *c->waits.ran_out = 0;
     return FLOCK_OK;
   });
   if (rc) {
     *out = nullptr;
+    if (c->st) cudaStreamDestroy(c->st);
     delete c;
     return rc;
   }
@@ -179,7 +174,11 @@ int flock_ctx_create(int device, uint64_t hbm_budget_bytes, flock_ctx** out) {
 void flock_ctx_destroy(flock_ctx* c) {
   if (!c) return;
   c->server.reset();  // joins the serving threads, frees their setups
-  if (c->st) cudaStreamDestroy(c->st);
+  if (c->st) {
+    cudaStreamSynchronize(c->st);  // (a call that failed may have left work that can still set the word)
+    cudaStreamDestroy(c->st);
+  }
+  flock::pinned_give(c->waits.ran_out, sizeof(unsigned));
   delete c;
 }
 
@@ -244,6 +243,7 @@ int flock_setup_set_wait_polls(flock_setup* s, uint32_t polls) {
 int flock_ctx_set_wait_polls(flock_ctx* c, uint32_t polls) {
   if (!c) return FLOCK_ERR_ARG;
   c->waits.polls = polls;
+  if (c->server) c->server->set_wait_polls(polls);
   return FLOCK_OK;
 }
 
@@ -673,7 +673,7 @@ int flock_pcs_commit(flock_ctx* c, const uint64_t* z_packed, uint32_t m, uint8_t
     merkle_build(pd->cw, pd->n_leaves, 64 * sizeof(f128), pd->tree, c->st);
     CK(cudaMemcpyAsync(root32, pd->tree + 8 * (2 * pd->n_leaves - 2), 32, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    check_device_timeouts();
+    check_waits(c->waits);
     *out = pd.release();
     return FLOCK_OK;
   });
@@ -1023,6 +1023,7 @@ int flock_serve_start(flock_ctx* c, int slots) {
       budget = free_b > ((size_t)4 << 30) ? free_b - ((size_t)4 << 30) : free_b / 2;
     }
     c->server.reset(new flock::Server(c->device, budget, slots));
+    c->server->set_wait_polls(c->waits.polls);
     return FLOCK_OK;
   });
 }
@@ -1168,7 +1169,7 @@ int flock_ntt_rs_encode(flock_ctx* c, const uint64_t* msg, uint32_t log_msg_pos,
     ntt_rs_encode(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, c->st, c->waits);
     CK(cudaMemcpyAsync(out, dc.p, nc * 16, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    check_device_timeouts();
+    check_waits(c->waits);
     return FLOCK_OK;
   });
 }
@@ -1185,7 +1186,7 @@ int flock_ntt_rs_encode_plan(flock_ctx* c, const uint64_t* msg, uint32_t log_msg
     ntt_rs_encode_plan(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, plan_index, c->st, c->waits);
     CK(cudaMemcpyAsync(out, dc.p, nc * 16, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    check_device_timeouts();
+    check_waits(c->waits);
     return FLOCK_OK;
   });
 }
@@ -1325,6 +1326,7 @@ int flock_bench_ntt(flock_ctx* c, uint32_t log_msg_pos, uint32_t lanes, uint32_t
     *ms = time_launches(c->st, iters, [&] {
       ntt_rs_encode(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, c->st, c->waits);
     });
+    check_waits(c->waits);
     return FLOCK_OK;
   });
 }
@@ -1355,6 +1357,7 @@ int flock_bench_ntt_plan(flock_ctx* c, uint32_t log_msg_pos, uint32_t lanes, uin
     *ms = time_launches(c->st, iters, [&] {
       ntt_rs_encode_plan(dm.p, dc.p, (int)log_msg_pos, (int)lanes, (int)rate, plan_index, c->st, c->waits);
     });
+    check_waits(c->waits);
     return FLOCK_OK;
   });
 }

@@ -176,16 +176,8 @@ struct MpCoeffs {
   f128 c[8];
 };
 
-// A word of mapped host memory that kernels with bounded waits set when a wait
-// ran out; check_device_timeouts throws then (after a synchronisation of the
-// work it asks about).
-struct DeviceTimeouts {
-  volatile unsigned* host;
-  unsigned* dev;
-};
-const DeviceTimeouts& device_timeouts();
-void check_device_timeouts();
-// What a launch's bounded waits take: the word they set when one ran out, and
+// What a launch's bounded waits take: the word they set when one ran out
+// (page-locked, of the setup or context that launches), and
 // after how many polls of an mbarrier one has (a poll suspends for up to 4 us, so
 // the default is a second, where microseconds are expected).  What the wait was
 // for is in flight still, so it is waited for kWaitPolls longer; the CTA then
@@ -196,6 +188,9 @@ struct WaitLimit {
   unsigned* ran_out = nullptr;
   unsigned polls = kWaitPolls;
 };
+// Throws if a wait of the launches with `w` ran out, and clears the word; after a
+// synchronisation of the work it asks about.
+void check_waits(const WaitLimit& w);
 
 // K0
 void launch_witness_seed(uint64_t seed, uint32_t log2, uint32_t n_blocks, uint32_t n_slots, f128* z, f128* a,
@@ -282,6 +277,7 @@ struct BatchJob {
   // first tile of this job in the launch of pass p: of the tensor-core
   // passes' launch for a kind-3 pass, of the other kinds' launch otherwise
   uint64_t tile0[kMaxBatchPasses], tile0t[kMaxBatchPasses];
+  unsigned* ran_out;  // the job's own word (WaitLimit)
   uint32_t* tree;     // Merkle tree over 2^log_d leaves of 1 KiB
   uint64_t n_leaves, leaf0;
   uint64_t par0[24];  // first node of this job in the launch of parent level k
@@ -293,9 +289,9 @@ void ntt_replicate_batch(const BatchJob* jobs, int n_jobs, uint64_t total, cudaS
 size_t ntt_pass_batch_smem(const NttPass& p);
 void ntt_pass_batch(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_tiles, size_t smem, int grid,
                     cudaStream_t s);
-// the jobs' kind-3 passes; max_R: the largest layer count among them
+// the jobs' kind-3 passes; max_R: the largest layer count among them; polls: WaitLimit
 void ntt_pass_batch_t(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_tiles, int max_R, int sms,
-                      cudaStream_t s, const WaitLimit& w);
+                      cudaStream_t s, unsigned polls);
 void merkle_leaves_batch(const BatchJob* jobs, int n_jobs, uint64_t total, cudaStream_t s);
 void merkle_parents_batch(const BatchJob* jobs, int n_jobs, int level, uint64_t total, cudaStream_t s);
 void merkle_top_batch(const BatchJob* jobs, int n_jobs, cudaStream_t s);

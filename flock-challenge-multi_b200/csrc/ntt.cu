@@ -452,16 +452,16 @@ struct TmapSetup {
     cta.taddr = __shfl_sync(0xffffffffu, *slot, 0);
     cta.rows = tm_rows(cta.mat);
   }
-  __device__ __forceinline__ void finish(const WaitLimit& w) {
-    if (tm_lds32(cta.dead())) {  // (set before the last tile's last barrier, if at all)
-      // products that were started before the thread that starts them saw the word
-      if (cta.warp == 0 && tm_elect()) tm_drain(cta.bar_end());
-      if (threadIdx.x == 0) *w.ran_out = 1;
-    }
+  // true: a wait ran out
+  __device__ __forceinline__ bool finish() {
+    const bool dead = tm_lds32(cta.dead());  // (set before the last tile's last barrier, if at all)
+    // products that were started before the thread that starts them saw the word
+    if (dead && cta.warp == 0 && tm_elect()) tm_drain(cta.bar_end());
     tm_store_done();
     tm_fence_before();
     __syncthreads();
     if (cta.warp == 0) tm_free(cta.taddr);
+    return dead;
   }
 };
 
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(128, 4) k_ntt_pass_t(PassArgs p, uint64_t n_ti
   uint64_t seq_hi = ~0ull;
   const uint64_t t0 = blockIdx.x * per, t1 = min(t0 + per, n_tiles);
   for (uint64_t t = t0; t < t1; t++) ntt_tile_t(p, t, S.seqs, S.cta, seq_hi, sh, w.polls);
-  S.finish(w);
+  if (S.finish() && threadIdx.x == 0) *w.ran_out = 1;
 }
 
 template <bool TRANSPOSE, int KIND>
@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(256, 2) k_ntt_pass_batch(const BatchJob* __res
 // The same for the jobs whose pass runs on the tensor cores.
 __global__ void __launch_bounds__(128, 4) k_ntt_pass_batch_t(const BatchJob* __restrict__ jobs, int n_jobs, int pass,
                                                              uint64_t total_tiles, uint64_t per, int max_R, TmShifts sh,
-                                                             WaitLimit w) {
+                                                             uint32_t polls) {
   extern __shared__ __align__(16) uint8_t raw[];
   TmapSetup S(raw, max_R);
   uint64_t seq_hi = ~0ull;
@@ -539,9 +539,12 @@ __global__ void __launch_bounds__(128, 4) k_ntt_pass_batch_t(const BatchJob* __r
     }
     if (lo != job) seq_hi = ~0ull;
     job = lo;
-    ntt_tile_t(a, t - J.tile0t[pass], S.seqs, S.cta, seq_hi, sh, w.polls);
+    ntt_tile_t(a, t - J.tile0t[pass], S.seqs, S.cta, seq_hi, sh, polls);
   }
-  S.finish(w);
+  if (S.finish())  // the jobs that had tiles here
+    for (int j = threadIdx.x; j < n_jobs; j += 128)
+      if (jobs[j].tile0t[pass] < t1 && (j + 1 < n_jobs ? jobs[j + 1].tile0t[pass] : total_tiles) > t0)
+        *jobs[j].ran_out = 1;
 }
 
 __global__ void k_replicate_batch(const BatchJob* __restrict__ jobs, int n_jobs, uint64_t total) {
@@ -964,13 +967,13 @@ void ntt_pass_batch(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_t
 }
 
 void ntt_pass_batch_t(const BatchJob* jobs, int n_jobs, int pass, uint64_t total_tiles, int max_R, int sms,
-                      cudaStream_t s, const WaitLimit& w) {
+                      cudaStream_t s, unsigned polls) {
   const size_t smem = pass_t_smem(max_R);
   CK(cudaFuncSetAttribute(k_ntt_pass_batch_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_t_smem(kMaxRt)));
   const uint64_t per = tiles_per_cta(total_tiles, sms);
   count_launch();
   k_ntt_pass_batch_t<<<(unsigned)((total_tiles + per - 1) / per), 128, smem, s>>>(
-      jobs, n_jobs, pass, total_tiles, per, max_R, tm_shifts(), w);
+      jobs, n_jobs, pass, total_tiles, per, max_R, tm_shifts(), polls);
 }
 
 NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaStream_t s, const WaitLimit& w,
@@ -995,7 +998,14 @@ NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaS
     k_fill_random<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(reinterpret_cast<uint64_t*>(scratch), words);
     CK(cudaGetLastError());
   }
-  cudaEvent_t e0, e1;
+  struct Events {
+    cudaEvent_t e[2] = {nullptr, nullptr};
+    ~Events() {
+      for (cudaEvent_t v : e)
+        if (v) cudaEventDestroy(v);
+    }
+  } events;
+  cudaEvent_t &e0 = events.e[0], &e1 = events.e[1];
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   // one warm launch, then the best of two timed launches (CUDA events on
@@ -1008,6 +1018,7 @@ NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaS
       launch_pass(ps, scratch, ev, log_d, lanes, false, s, w);
       CK(cudaEventRecord(e1, s));
       CK(cudaEventSynchronize(e1));
+      check_waits(w);  // the time of a pass that gave up is no time
       float t = 0;
       CK(cudaEventElapsedTime(&t, e0, e1));
       best = std::min(best, t);
@@ -1055,8 +1066,6 @@ NttPlan ntt_autotune(f128* scratch, int log_d, int lanes, int layer_begin, cudaS
     }
     if (total < best_total) { best_total = total; best_plan = plan; }
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   std::lock_guard<std::mutex> lk(g_plan_mu);
   tuned_plans()[key] = best_plan;
   if (best_ms) *best_ms = best_total;

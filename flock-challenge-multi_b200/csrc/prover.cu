@@ -37,6 +37,7 @@ T* dalloc(size_t n, cudaStream_t st) {
 // Page-locked host blocks are recycled rather than freed, for the same reason.
 std::mutex g_pin_mu;
 std::multimap<size_t, void*> g_pin_free;
+}  // namespace
 void* pinned_take(size_t bytes) {
   {
     std::lock_guard<std::mutex> lk(g_pin_mu);
@@ -56,8 +57,6 @@ void pinned_give(void* p, size_t bytes) {
   std::lock_guard<std::mutex> lk(g_pin_mu);
   g_pin_free.emplace(bytes, p);
 }
-
-}  // namespace
 
 // ---------------------------------------------------------------- setup --
 size_t Setup::estimate_bytes(uint32_t log2, int hash) {
@@ -121,10 +120,11 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   idx = dalloc<uint64_t>(1 << 16, st);
   gather = dalloc<f128>(1 << 16, st);
   d_found = dalloc<unsigned long long>(1, st);
-  mail_block = pinned_take(kMailBytes);
+  mail_block = pinned_take(kMailBytes + sizeof(unsigned));
   d_ticket = dalloc<unsigned>(1, st);
   mail = mailbox_at(mail_block, d_ticket);
-  waits.ran_out = device_timeouts().dev;
+  waits.ran_out = reinterpret_cast<unsigned*>(static_cast<uint8_t*>(mail_block) + kMailBytes);
+  *waits.ran_out = 0;
   h_out = static_cast<f128*>(pinned_take(1024 * sizeof(f128)));
   h_stage = static_cast<uint8_t*>(pinned_take(kStageBytes));
   const Statement& S = statement(hash);
@@ -239,6 +239,7 @@ BatchCommit batch_commit_async(const std::vector<Setup*>& setups, const std::vec
     b.cw = S.cw0;
     b.log_d = S.m - 12;
     b.ev = ntt_evals(b.log_d);
+    b.ran_out = S.waits.ran_out;
     b.msg_len = S.n_words;
     b.rep0 = rep;
     rep += b.msg_len;
@@ -294,7 +295,7 @@ BatchCommit batch_commit_async(const std::vector<Setup*>& setups, const std::vec
       // pass 0 reads each job's message as its replicated codeword
       for (int p = 0; p < max_pass; p++) {
         if (tiles[p]) ntt_pass_batch(dj, n, p, tiles[p], smem, 2 * sms, st);
-        if (tiles_t[p]) ntt_pass_batch_t(dj, n, p, tiles_t[p], max_R, sms, st, setups[0]->waits);
+        if (tiles_t[p]) ntt_pass_batch_t(dj, n, p, tiles_t[p], max_R, sms, st, setups[0]->waits.polls);
       }
       merkle_leaves_batch(dj, n, leaves, st);
       for (int l = 1; l <= max_level; l++) merkle_parents_batch(dj, n, l, par[l], st);
@@ -339,7 +340,7 @@ Setup::~Setup() {
     if (L.cw) cudaFreeAsync(L.cw, st);
     if (L.tree) cudaFreeAsync(L.tree, st);
   }
-  pinned_give(mail_block, kMailBytes);
+  pinned_give(mail_block, kMailBytes + sizeof(unsigned));
   pinned_give(h_out, 1024 * sizeof(f128));
   pinned_give(h_stage, kStageBytes);
   for (auto g : commit_graph)
@@ -474,6 +475,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   P.merkle_fn = merkle_fn;
   pending_.clear();  // (left over only by a proof that threw)
   stage_off_ = 0;
+  if (!committed) *waits.ran_out = 0;  // (likewise; batch_commit may have set it for this proof)
   const int gs = grid_sms > 0 && grid_sms < sms ? grid_sms : sms;
   const int G = gs * 4;
   const uint32_t n_slots = 1u << n_log;
@@ -1177,7 +1179,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
   }
   mark(9);
   CK(cudaStreamSynchronize(st));
-  check_device_timeouts();
+  check_waits(waits);
   finish_openings();
   std::vector<uint8_t> bytes = encode(P);
   return bytes;

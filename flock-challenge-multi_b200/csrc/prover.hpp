@@ -10,6 +10,10 @@
 
 namespace flock {
 
+// Page-locked host blocks, recycled by size rather than freed (cudaFreeHost waits
+// for the whole device).
+void* pinned_take(size_t bytes);
+void pinned_give(void* p, size_t bytes);
 void scatter(f128* dst, const uint64_t* pos, const f128* vals, size_t n, cudaStream_t s);
 class Setup;
 // Fused witness + commit of several seeded proofs (one graph of batched

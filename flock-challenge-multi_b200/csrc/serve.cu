@@ -94,6 +94,7 @@ std::vector<JobResult> Server::prove_batch(const std::vector<BatchItem>& jobs, i
     // one group overlaps the transcript phases of the earlier ones.
     constexpr size_t kGroup = 8;
     const size_t nw = wave.size();
+    for (auto& w : wave) w.second->waits.polls = polls_;
     std::unique_ptr<std::atomic<int>[]> ready(new std::atomic<int>[nw]);  // 0 wait, 1 go, 2 commit failed
     std::vector<std::string> commit_err(nw);
     std::vector<size_t> seeded;
@@ -324,6 +325,7 @@ void Server::worker(bool small_only) {
       r.error = e.what();
     }
     if (stop_ && !s) return;
+    if (s) s->waits.polls = polls_;
     if (s) s->grid_sms = n_slots_ >= 3 && job.log2 > kSmallLog2 ? s->sms - kReservedSms : 0;
     const auto t_run = Clock::now();
     if (s) {

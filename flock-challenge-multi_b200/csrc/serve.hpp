@@ -73,6 +73,8 @@ class Server {
   // self-check: verify every proof on its own setup before returning it; a
   // proof that fails gets FLOCK_ERR_VERIFY and the failed check's name
   void set_verify(bool on) { verify_ = on; }
+  // WaitLimit::polls of the proofs started from now on
+  void set_wait_polls(unsigned polls) { polls_ = polls; }
   int slots() const { return n_slots_; }
   uint64_t budget() const { return budget_; }
   uint64_t cached_bytes();
@@ -119,6 +121,7 @@ class Server {
   uint64_t next_ticket_ = 1, use_clock_ = 0;
   bool stop_ = false;
   std::atomic<bool> verify_{false};
+  std::atomic<unsigned> polls_{kWaitPolls};
   int n_slots_ = 0;  // set before the slot threads start (they read it)
   std::vector<std::thread> workers_;
   std::mutex batch_mu_;  // one batch at a time

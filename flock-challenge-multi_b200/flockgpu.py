@@ -406,7 +406,7 @@ class Context:
             pass
 
     def set_wait_polls(self, polls: int) -> None:
-        """The limit of the bounded waits of the kernels that this context's own calls launch."""
+        """The limit of the bounded waits of the kernels that this context's calls launch (its Provers' calls have their own)."""
         self._check(self.lib.flock_ctx_set_wait_polls(self.h, polls), "ctx_set_wait_polls")
 
     # ---- serving (continuous batching of proof jobs) ----

@@ -128,8 +128,8 @@ int flock_ctx_set_transcript(flock_ctx* ctx, int hash);
  * copies or tensor-core products; the call that launched it then returns
  * FLOCK_ERR_CUDA.  Default 2^18, a second where microseconds are expected.  With 0 the kernels start nothing that they wait for, so that each
  * first wait runs out (how the error path is tested).  Of a setup's proofs (their
- * captured commitment keeps the default) / of the context's own calls.  Not while
- * one of them runs. */
+ * captured commitment keeps the default) / of the context's other calls, its
+ * served and batched proofs among them.  Not while one of them runs. */
 int flock_setup_set_wait_polls(flock_setup* s, uint32_t polls);
 int flock_ctx_set_wait_polls(flock_ctx* ctx, uint32_t polls);
 
