@@ -234,6 +234,8 @@ int flock_ctx_set_transcript(flock_ctx* c, int hash) {
   return FLOCK_OK;
 }
 
+uint64_t flock_setup_device_bytes(flock_setup* s) { return s ? s->s->device_bytes : 0; }
+
 int flock_setup_set_wait_polls(flock_setup* s, uint32_t polls) {
   if (!s) return FLOCK_ERR_ARG;
   s->s->waits.polls = polls;

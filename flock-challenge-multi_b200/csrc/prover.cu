@@ -149,8 +149,11 @@ Setup::Setup(int device, uint32_t log2_, int stream_priority, int hash_, int mer
   tune_ntt_plans();
   capture_commit();
   CK(cudaStreamSynchronize(st));  // the buffers exist for every stream from here on
-  // the driver's share: captured graphs, events, the stream
-  device_bytes = t_alloc_bytes - bytes0 + ((size_t)1 << 20);
+  // whole pages of device memory; what the driver keeps for the stream, events
+  // and graphs is in the last one's rest (building setups of 2^8 to 2^14 took
+  // the device the pool's growth and none or one page more)
+  constexpr size_t kPage = (size_t)2 << 20;
+  device_bytes = (t_alloc_bytes - bytes0 + kPage - 1) / kPage * kPage;
 }
 
 // Tune the pass plans of every NTT shape a proof of this size runs, on this

@@ -147,7 +147,7 @@ class Setup {
   // device bytes a setup for 2^log2 compressions holds (an upper estimate,
   // used for admission before allocating)
   static size_t estimate_bytes(uint32_t log2, int hash = kHashBlake3);
-  size_t device_bytes = 0;  // allocated by the constructor
+  size_t device_bytes = 0;  // allocated by the constructor, in whole pages of 2 MiB
 
   friend BatchCommit batch_commit_async(const std::vector<Setup*>& setups, const std::vector<uint64_t>& seeds,
                                         cudaStream_t st);

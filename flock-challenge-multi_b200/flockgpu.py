@@ -44,7 +44,7 @@ EXPORTS = (
     "flock_zerocheck_round1_deg4", "flock_bench_round1_deg4", "flock_keccak3_setup_create",
     "flock_keccak3_verify_bundle", "flock_keccak3_statement_digest", "flock_keccak3_witness", "flock_keccak3_comb",
     "flock_sha256_prove_chain", "flock_sha256_chain_blocks", "flock_keccak_prove_chain", "flock_keccak_chain_states",
-    "flock_setup_set_wait_polls", "flock_ctx_set_wait_polls",
+    "flock_setup_set_wait_polls", "flock_ctx_set_wait_polls", "flock_setup_device_bytes",
 )
 # the hash behind Merkle trees / the transcript (HashKind discriminants)
 HASH = {"sha256": 0, "blake3": 1}
@@ -127,6 +127,8 @@ def load() -> ctypes.CDLL:
                                           ctypes.POINTER(u64)]
         lib.flock_merkle_root_noalloc.argtypes = [vp, sz, sz, vp, vp]
         lib.flock_setup_set_wait_polls.argtypes = [vp, u32]
+        lib.flock_setup_device_bytes.argtypes = [vp]
+        lib.flock_setup_device_bytes.restype = u64
         lib.flock_ctx_set_wait_polls.argtypes = [vp, u32]
         lib.flock_serve_start.argtypes = [vp, i32]
         lib.flock_serve_prewarm.argtypes = [vp, u32, i32, ctypes.POINTER(i32)]
@@ -968,6 +970,10 @@ class Prover:
             self.close()
         except Exception:
             pass
+
+    def device_bytes(self) -> int:
+        """Device memory of the setup's buffers, in whole pages (what serving budgets by)."""
+        return self.ctx.lib.flock_setup_device_bytes(self.h)
 
     def set_wait_polls(self, polls: int) -> None:
         """The limit of the bounded waits of the kernels of this setup's proofs."""

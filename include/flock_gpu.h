@@ -117,6 +117,9 @@ int flock_setup_create(flock_ctx* ctx, uint32_t log2_n, int hash, int profile, f
  * below that, FLOCK_ERR_ARG here). */
 int flock_setup_create_blocks(flock_ctx* ctx, size_t n_blocks, int hash, int profile, flock_setup** out);
 void flock_setup_destroy(flock_setup* s);
+/* Device memory of the setup's own buffers, in whole pages of 2 MiB: what it
+ * counts against a context's HBM budget while it is cached for serving. */
+uint64_t flock_setup_device_bytes(flock_setup* s);
 /* The transcript of this setup's proofs and of flock_verify on it:
  * FsChallenger::with_hash(domain, hash) (challenger.rs:227-250; SHA-256:
  * squeezes SHA256(state || ctr), PoW SHA256(digest || nonce)). */
