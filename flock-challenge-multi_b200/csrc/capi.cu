@@ -654,6 +654,36 @@ int flock_keccak3_comb(flock_ctx* c, const uint64_t* e, const uint64_t* alpha, c
   return keccak_comb_call(c, 3, e, alpha, beta, comb);
 }
 
+int flock_lincheck_comb(flock_ctx* c, int statement, const uint64_t* e, const uint64_t* alpha, const uint64_t* beta,
+                        uint32_t sms, uint64_t* comb, uint32_t* ctas) {
+  if (!c || !e || !alpha || !beta || !comb || !ctas || sms < 1 || (int)sms > c->sms ||
+      (statement != flock::kHashBlake3 && statement != flock::kHashSha256))
+    return FLOCK_ERR_ARG;
+  return guard(c, [&] {
+    const flock::Statement& S = flock::statement(statement);
+    const size_t kk = (size_t)1 << S.k_log;
+    DevBuf<uint32_t> ap(S.at_ptr.size()), bp(S.bt_ptr.size());
+    DevBuf<uint16_t> ar(S.at_row.size()), br(S.bt_row.size());
+    DevBuf<f128> de(kk), dc(2 * kk);
+    auto up = [&](auto& dst, const auto& src) {
+      CK(cudaMemcpyAsync(dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice, c->st));
+    };
+    up(ap, S.at_ptr);
+    up(bp, S.bt_ptr);
+    up(ar, S.at_row);
+    up(br, S.bt_row);
+    CK(cudaMemcpyAsync(de.p, e, kk * 16, cudaMemcpyHostToDevice, c->st));
+    int n = 0;
+    lc_comb(ap.p, ar.p, bp.p, br.p, de.p, mk(alpha[0], alpha[1]), mk(beta[0], beta[1]), S.z_const, (int)kk, dc.p,
+            (int)sms, c->st, &n);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(comb, dc.p, kk * 16, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    *ctas = (uint32_t)n;
+    return FLOCK_OK;
+  });
+}
+
 int flock_pcs_commit(flock_ctx* c, const uint64_t* z_packed, uint32_t m, uint8_t* root32, flock_prover_data** out) {
   if (!c || !z_packed || !root32 || !out) return FLOCK_ERR_ARG;
   if (m < 22 || m > 34) {

@@ -777,7 +777,7 @@ std::vector<uint8_t> Setup::prove(const uint64_t* seed, const uint32_t* blocks_d
     eq_build(x_inner.data(), (int)x_inner.size(), hone(), zv_pre, st);
     outer64(L.data(), zv_pre, (size_t)1 << x_inner.size(), eq_inner, st);
     if (is_keccak(hash)) keccak_comb(eq_inner, alpha, beta, kc_masks, kc_w, comb, st, keccak_width(hash));
-    else lc_comb(at_ptr, at_row, bt_ptr, bt_row, eq_inner, alpha, beta, statement(hash).z_const, kk, comb, st);
+    else lc_comb(at_ptr, at_row, bt_ptr, bt_row, eq_inner, alpha, beta, statement(hash).z_const, kk, comb, gs, st);
     eq_table(x_outer, scratch_eq());
     CK(cudaMemsetAsync(zv, 0, kk * sizeof(f128), st));
     lc_zvec(z, scratch_eq(), (size_t)1 << (m - k_log), k_log, zv, gs, st, waits);

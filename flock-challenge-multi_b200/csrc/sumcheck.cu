@@ -243,14 +243,14 @@ __global__ void __launch_bounds__(256) k_lc_round_quad(f128* comb, f128* zv, int
 }
 
 void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_ptr, const uint16_t* bt_row,
-             const f128* eq, f128 alpha, f128 beta, int pin, int k, f128* comb, cudaStream_t s) {
+             const f128* eq, f128 alpha, f128 beta, int pin, int k, f128* comb, int sms, cudaStream_t s,
+             int* ctas) {
   const int parts = k <= (1 << 14) ? 2 : 4;
   const size_t smem = (size_t)k * 16 / parts;
   if (smem > ((size_t)128 << 10)) throw CudaError("lc_comb: at most 2^15 rows");
-  int dev = 0, sms = 0;
-  CK(cudaGetDevice(&dev));
-  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const dim3 grid(sms / parts, parts);
+  // one CTA fits an SM, and it stays for the whole launch
+  const dim3 grid(std::max(1, sms / parts), parts);
+  if (ctas) *ctas = (int)(grid.x * grid.y);
   count_launch(2);
   if (parts == 2) {
     CK(cudaFuncSetAttribute(k_lc_sums<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 << 10));

@@ -893,15 +893,17 @@ std::string verify_bundle(const uint8_t* bytes, size_t len, const std::string& d
 // The device half of the verifier: the lincheck's matrix combination over
 // this setup's CSC copy of the block matrices, with the prover's kernels.
 namespace {
-// Device scratch of one verification in flight: eq(x_inner) (256 values), the
-// lincheck's eq table and matrix combination (2^14 values each), the opened
-// rows (1 MiB) and their leaf chaining values (512 KiB).
+// Device scratch of one verification in flight: eq(x_inner) (2^(k_log - 6)
+// values), the lincheck's eq table (2^k_log) and matrix combination (twice that,
+// for its column sums), the opened rows (1 MiB) and their leaf chaining values
+// (512 KiB).
 struct VerifyBufs {
   f128 *eqx, *eqi, *comb;
   f128* kcw;  // the Keccak walker's W rows (Keccak statements only)
   uint8_t* rows;
   uint32_t* cvs;
   size_t rows_cap, cvs_cap;  // bytes
+  int sms;                   // that a launch may fill
 };
 // the device half of the verifier over the CSC copy of the block matrices
 // given by at_*, bt_* (the Keccak statement's implicit matrices by its
@@ -924,7 +926,7 @@ VerifyStatement device_statement(int m, int hash, const std::array<uint8_t, 32>&
       CK(cudaGetDevice(&dev));
       keccak_comb(B.eqi, alpha, beta, keccak_masks(dev), B.kcw, B.comb, st, keccak_width(hash));
     } else {
-      lc_comb(at_ptr, at_row, bt_ptr, bt_row, B.eqi, alpha, beta, pin, kk, B.comb, st);
+      lc_comb(at_ptr, at_row, bt_ptr, bt_row, B.eqi, alpha, beta, pin, kk, B.comb, B.sms, st);
     }
     CK(cudaMemcpyAsync(cv.data(), B.comb, kk * sizeof(f128), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -981,7 +983,8 @@ const DevCsc& shared_csc(int device, int hash) {
 // The setup's own buffers and stream (flock_verify: the caller owns the setup).
 std::string Setup::verify(const uint8_t* bytes, size_t len, const std::string& domain, const MerklePublic* merkle) {
   VerifyBufs B{zv_pre, eq_inner, comb, kc_w, reinterpret_cast<uint8_t*>(gather), reinterpret_cast<uint32_t*>(idx),
-               ((size_t)1 << 16) * sizeof(f128), ((size_t)1 << 16) * sizeof(uint64_t)};
+               ((size_t)1 << 16) * sizeof(f128), ((size_t)1 << 16) * sizeof(uint64_t),
+               grid_sms > 0 && grid_sms < sms ? grid_sms : sms};
   if (merkle && hash != kHashSha256) return "a Merkle path is a SHA-256 statement";
   VerifyStatement V = device_statement(m, hash, digest, at_ptr, at_row, bt_ptr, bt_row, B, st);
   V.merkle = merkle;
@@ -991,6 +994,7 @@ std::string Setup::verify(const uint8_t* bytes, size_t len, const std::string& d
 
 Verifier::Verifier(int device) : device_(device) {
   DeviceScope on(device);
+  CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device));
   CK(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
   CK(cudaMalloc(&eqx_, ((size_t)1 << (kMaxKLog - kKSkip)) * sizeof(f128)));  // eq(x_inner), 2^(k_log - 6)
   CK(cudaMalloc(&eqi_, ((size_t)1 << kMaxKLog) * sizeof(f128)));  // the largest block of the statements
@@ -1029,7 +1033,7 @@ std::string Verifier::verify(const uint8_t* bytes, size_t len, const std::string
   // thread has current; the caller's device is restored on return
   DeviceScope on(device_);
   const DevCsc& C = shared_csc(device_, hash);
-  const VerifyBufs B{eqx_, eqi_, comb_, kcw_, rows_, cvs_, kRowsCap, kCvsCap};
+  const VerifyBufs B{eqx_, eqi_, comb_, kcw_, rows_, cvs_, kRowsCap, kCvsCap, sms_};
   VerifyStatement V = device_statement((int)mm, hash, statement_digest(hash, (int)mm), C.at_ptr, C.at_row, C.bt_ptr,
                                        C.bt_row, B, st_);
   V.merkle = merkle;

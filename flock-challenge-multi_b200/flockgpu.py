@@ -45,6 +45,7 @@ EXPORTS = (
     "flock_keccak3_verify_bundle", "flock_keccak3_statement_digest", "flock_keccak3_witness", "flock_keccak3_comb",
     "flock_sha256_prove_chain", "flock_sha256_chain_blocks", "flock_keccak_prove_chain", "flock_keccak_chain_states",
     "flock_setup_set_wait_polls", "flock_ctx_set_wait_polls", "flock_setup_device_bytes",
+    "flock_lincheck_comb",
 )
 # the hash behind Merkle trees / the transcript (HashKind discriminants)
 HASH = {"sha256": 0, "blake3": 1}
@@ -128,6 +129,7 @@ def load() -> ctypes.CDLL:
         lib.flock_merkle_root_noalloc.argtypes = [vp, sz, sz, vp, vp]
         lib.flock_setup_set_wait_polls.argtypes = [vp, u32]
         lib.flock_setup_device_bytes.argtypes = [vp]
+        lib.flock_lincheck_comb.argtypes = [vp, i32, vp, vp, vp, u32, vp, ctypes.POINTER(u32)]
         lib.flock_setup_device_bytes.restype = u64
         lib.flock_ctx_set_wait_polls.argtypes = [vp, u32]
         lib.flock_serve_start.argtypes = [vp, i32]
@@ -490,6 +492,17 @@ class Context:
         self._check(getattr(self.lib, f"flock_keccak{_kw(width)}_witness")(
             self.h, _ptr(states), states.shape[0], n_log, _ptr(z), _ptr(a), _ptr(b)), "keccak_witness")
         return z, a, b
+
+    def lincheck_comb(self, statement: str, e: np.ndarray, alpha, beta, sms: int):
+        """(alpha A^T e + B^T e + beta [const] of the statement's block matrices as (2^k_log, 2)
+        u64, CTAs of the column sums), the sums on at most `sms` SMs."""
+        e = np.ascontiguousarray(e, np.uint64)
+        assert e.size == 2 << {"blake3": 14, "sha256": 15}[statement]
+        al, be = (np.array(v, np.uint64) for v in (alpha, beta))
+        out, n = np.zeros(e.size, np.uint64), ctypes.c_uint32()
+        self._check(self.lib.flock_lincheck_comb(self.h, {"blake3": 0, "sha256": 1}[statement], _ptr(e), _ptr(al),
+                                                 _ptr(be), sms, _ptr(out), ctypes.byref(n)), "lincheck_comb")
+        return out.reshape(-1, 2), n.value
 
     def keccak_comb(self, e: np.ndarray, alpha, beta, width: int = 1) -> np.ndarray:
         """The Keccak lincheck's alpha A^T e + B^T e + beta [const] on the GPU

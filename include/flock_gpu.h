@@ -323,6 +323,11 @@ int flock_keccak_witness(flock_ctx* ctx, const flock_keccak_state* states, size_
  * [const] over the 2^16 rows of a block, on the GPU (e, comb: 2^16 F128 as
  * lo, hi u64 pairs; alpha, beta: one F128). */
 int flock_keccak_comb(flock_ctx* ctx, const uint64_t* e, const uint64_t* alpha, const uint64_t* beta, uint64_t* comb);
+/* Debug/test: the same combination of a stored statement's block matrices
+ * (statement 0: BLAKE3, 2^14 rows; 1: SHA-256, 2^15), its column sums on at most
+ * `sms` SMs in *ctas CTAs, one an SM. */
+int flock_lincheck_comb(flock_ctx* ctx, int statement, const uint64_t* e, const uint64_t* alpha, const uint64_t* beta,
+                        uint32_t sms, uint64_t* comb, uint32_t* ctas);
 /* KeccakSetup::prove_chain (keccak.rs:1000-1022) + ChainProofBundleLigerito
  * (hash_kind Keccak) bytes: the n states (n = the setup's n_keccaks, a power
  * of two: a chain fills every slot) form a chain state[i + 1] =
@@ -392,7 +397,7 @@ int flock_chain_blocks(uint64_t seed, const uint32_t* initial_cv, size_t steps, 
 int flock_verify(flock_setup* s, const uint8_t* bytes, size_t len, const uint8_t* domain, size_t dlen);
 /* The same verification without a prover setup, for any supported size
  * (2^8..2^20 compressions, read from the bundle): a verifier held by the
- * context and created on first use, with about 2 MiB of device scratch, plus
+ * context and created on first use, with 8 MiB of device scratch, plus
  * one device copy of the block matrices per device (about 45 MB, kept until
  * the process exits).  Calls on one context are serialised. */
 int flock_verify_bundle(flock_ctx* ctx, const uint8_t* bytes, size_t len, const uint8_t* domain, size_t dlen);
