@@ -684,6 +684,25 @@ int flock_lincheck_comb(flock_ctx* c, int statement, const uint64_t* e, const ui
   });
 }
 
+int flock_lincheck_fold(flock_ctx* c, const uint64_t* z, const uint64_t* eq, size_t n, uint32_t k_log, uint32_t sms,
+                        uint64_t* zv) {
+  if (!c || !z || !eq || !zv || !n || sms < 1 || (int)sms > c->sms || k_log > 17 || !lc_zvec_fits(n, (int)k_log))
+    return FLOCK_ERR_ARG;
+  return guard(c, [&] {
+    const size_t kk = (size_t)1 << k_log;
+    DevBuf<f128> dz(n * kk / 128), de(n), dv(kk);
+    CK(cudaMemcpyAsync(dz.p, z, n * kk / 8, cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(de.p, eq, n * 16, cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemsetAsync(dv.p, 0, kk * 16, c->st));
+    lc_zvec(dz.p, de.p, n, (int)k_log, dv.p, (int)sms, c->st, c->waits);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(zv, dv.p, kk * 16, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    check_waits(c->waits);
+    return FLOCK_OK;
+  });
+}
+
 int flock_pcs_commit(flock_ctx* c, const uint64_t* z_packed, uint32_t m, uint8_t* root32, flock_prover_data** out) {
   if (!c || !z_packed || !root32 || !out) return FLOCK_ERR_ARG;
   if (m < 22 || m > 34) {

@@ -346,6 +346,7 @@ void fold_pair_final(const f128* a_in, const f128* b_in, f128 rho, f128* out, cu
 void lc_comb(const uint32_t* at_ptr, const uint16_t* at_row, const uint32_t* bt_ptr, const uint16_t* bt_row,
              const f128* eq, f128 alpha, f128 beta, int pin, int k, f128* comb, int sms, cudaStream_t s,
              int* ctas = nullptr);
+bool lc_zvec_fits(size_t n_outer, int k_log);
 void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s,
              const WaitLimit& w);
 void lc_round(f128* comb, f128* zv, int len, bool fold, f128 r, bool emit, f128* out, cudaStream_t s,

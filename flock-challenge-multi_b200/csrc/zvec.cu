@@ -209,18 +209,26 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lc_zvec(GemmArgs G, WaitLim
 
 }  // namespace
 
+static uint64_t fold_steps(size_t n_outer, int k_log) {
+  return (uint64_t)((n_outer + kRowsStep - 1) / kRowsStep) << (k_log - 8);
+}
+// the kernel counts rows and steps in 32 bits
+bool lc_zvec_fits(size_t n_outer, int k_log) {
+  return k_log >= 8 && k_log <= 17 && !(n_outer >> 30) && !(fold_steps(n_outer, k_log) >> 32);
+}
+
 // zv[i] ^= XOR over o < n_outer with bit i of o's 2^k_log-bit block set of eqo[o]
 // (sms: the SMs the launch may fill, one wave of resident CTAs on them)
 void lc_zvec(const f128* z, const f128* eqo, size_t n_outer, int k_log, f128* zv, int sms, cudaStream_t s,
              const WaitLimit& w) {
   if (!w.ran_out) throw CudaError("lc_zvec: a word for its waits");
-  if (k_log < 8 || k_log > 17 || n_outer >> 30) throw CudaError("lc_zvec: bad shape");
+  if (!lc_zvec_fits(n_outer, k_log)) throw CudaError("lc_zvec: bad shape");
+  if (!n_outer) return;
   GemmArgs G{reinterpret_cast<const uint32_t*>(z), 1u << (k_log - 5), (uint32_t)n_outer, 1u << (k_log - 8),
              reinterpret_cast<const uint32_t*>(eqo), zv};
   CK(cudaFuncSetAttribute(k_lc_zvec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
-  const uint64_t steps = (uint64_t)((G.n_rows + kRowsStep - 1) / kRowsStep) * G.cols;
   const uint64_t grid = (uint64_t)resident_grid((const void*)k_lc_zvec, kGemmThreads, kGemmSmem, sms);
   count_launch();
-  k_lc_zvec<<<(unsigned)std::max<uint64_t>(1, std::min(grid, steps)), kGemmThreads, kGemmSmem, s>>>(
+  k_lc_zvec<<<(unsigned)std::max<uint64_t>(1, std::min(grid, fold_steps(n_outer, k_log))), kGemmThreads, kGemmSmem, s>>>(
       G, w);
 }

@@ -45,7 +45,7 @@ EXPORTS = (
     "flock_keccak3_verify_bundle", "flock_keccak3_statement_digest", "flock_keccak3_witness", "flock_keccak3_comb",
     "flock_sha256_prove_chain", "flock_sha256_chain_blocks", "flock_keccak_prove_chain", "flock_keccak_chain_states",
     "flock_setup_set_wait_polls", "flock_ctx_set_wait_polls", "flock_setup_device_bytes",
-    "flock_lincheck_comb",
+    "flock_lincheck_comb", "flock_lincheck_fold",
 )
 # the hash behind Merkle trees / the transcript (HashKind discriminants)
 HASH = {"sha256": 0, "blake3": 1}
@@ -129,6 +129,7 @@ def load() -> ctypes.CDLL:
         lib.flock_merkle_root_noalloc.argtypes = [vp, sz, sz, vp, vp]
         lib.flock_setup_set_wait_polls.argtypes = [vp, u32]
         lib.flock_setup_device_bytes.argtypes = [vp]
+        lib.flock_lincheck_fold.argtypes = [vp, vp, vp, sz, u32, u32, vp]
         lib.flock_lincheck_comb.argtypes = [vp, i32, vp, vp, vp, u32, vp, ctypes.POINTER(u32)]
         lib.flock_setup_device_bytes.restype = u64
         lib.flock_ctx_set_wait_polls.argtypes = [vp, u32]
@@ -492,6 +493,15 @@ class Context:
         self._check(getattr(self.lib, f"flock_keccak{_kw(width)}_witness")(
             self.h, _ptr(states), states.shape[0], n_log, _ptr(z), _ptr(a), _ptr(b)), "keccak_witness")
         return z, a, b
+
+    def lincheck_fold(self, z: np.ndarray, eq: np.ndarray, k_log: int, sms: int) -> np.ndarray:
+        """XOR of eq[o] over the blocks o (rows of z, 2^k_log bits) with bit i set, for each i: (2^k_log, 2) u64."""
+        z, eq = np.ascontiguousarray(z, np.uint64), np.ascontiguousarray(eq, np.uint64)
+        n = eq.size // 2
+        assert z.size == n << (k_log - 6)
+        out = np.zeros((1 << k_log, 2), np.uint64)
+        self._check(self.lib.flock_lincheck_fold(self.h, _ptr(z), _ptr(eq), n, k_log, sms, _ptr(out)), "lincheck_fold")
+        return out
 
     def lincheck_comb(self, statement: str, e: np.ndarray, alpha, beta, sms: int):
         """(alpha A^T e + B^T e + beta [const] of the statement's block matrices as (2^k_log, 2)

@@ -328,6 +328,10 @@ int flock_keccak_comb(flock_ctx* ctx, const uint64_t* e, const uint64_t* alpha, 
  * `sms` SMs in *ctas CTAs, one an SM. */
 int flock_lincheck_comb(flock_ctx* ctx, int statement, const uint64_t* e, const uint64_t* alpha, const uint64_t* beta,
                         uint32_t sms, uint64_t* comb, uint32_t* ctas);
+/* Debug/test: the lincheck's block fold: zv[i] = XOR of eq[o] over the n blocks o
+ * of 2^k_log bits (8 <= k_log <= 17) whose bit i is set, on at most `sms` SMs. */
+int flock_lincheck_fold(flock_ctx* ctx, const uint64_t* z, const uint64_t* eq, size_t n, uint32_t k_log, uint32_t sms,
+                        uint64_t* zv);
 /* KeccakSetup::prove_chain (keccak.rs:1000-1022) + ChainProofBundleLigerito
  * (hash_kind Keccak) bytes: the n states (n = the setup's n_keccaks, a power
  * of two: a chain fills every slot) form a chain state[i + 1] =
