@@ -834,7 +834,10 @@ void launch_pass(const NttPass& ps, f128* data, const f128* ev, int log_d, int l
     if (transpose) throw CudaError("ntt: tensor passes run forward only");
     if (!w.ran_out) throw CudaError("ntt: a tensor pass needs a word for its waits");
     CK(cudaFuncSetAttribute(k_ntt_pass_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_t_smem(kMaxRt)));
-    const uint64_t per = tiles_per_cta(tiles, 148);
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const uint64_t per = tiles_per_cta(tiles, sms);
     count_launch();
     k_ntt_pass_t<<<(unsigned)((tiles + per - 1) / per), 128, pass_t_smem(ps.R), s>>>(a, tiles, per, tm_shifts(), w);
     return;
