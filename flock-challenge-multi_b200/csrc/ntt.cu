@@ -275,10 +275,11 @@ __device__ __forceinline__ void ntt_tile_w(const PassArgs& p, uint64_t t_id, f12
 // Bound: the integer pipe (spreading and merging bits, 96 of about 160 of its
 // operations a product; writing matrices 40 more), then the dependent chain of
 // a unit, which four CTAs do not quite cover.  Measured, 2^20 positions x 64
-// lanes: 7.44 ms, 8.6 10^10 products/s, against 11.80 ms for the table passes
+// lanes: 7.49 ms, 8.5 10^10 products/s, against 11.80 ms for the table passes
 // (their ceiling, the shared-memory pipe, is 7.27 10^10) and 17.9 ms for the
-// integer products; 2^16: 0.479 / 0.611 / 0.914 ms; 2^12: 0.049 / 0.070 /
-// 0.064 ms.  R = 4 throughout (more passes, fewer matrices) takes 8.27 ms.
+// integer products; 2^16: 0.477 / 0.611 / 0.914 ms; 2^12: 0.046 / 0.070 /
+// 0.064 ms.  R = 4 throughout (one pass more, and 15 matrices for 16 units in
+// place of 31 for 40) takes 8.27 ms.
 constexpr int kMaxRt = 5;
 size_t pass_t_smem(int R) {
   return 1024 + 2 * kTmMatBytes + ((size_t)64 << R) * sizeof(f128) + ((size_t)1 << R) * 48 + 64;
@@ -785,8 +786,8 @@ std::vector<std::vector<std::pair<int, int>>> candidate_splits_t(int lanes, int 
 
 // From 2^kTensorMinLog positions on there are tiles enough for the SMs and the
 // tensor-core passes are the fastest of all kinds (2^12 positions x 64 lanes:
-// 0.049 ms against 0.057 ms for the best mix of the others; 2^14: 0.121 / 0.167;
-// 2^20: 7.44 / 11.8 ms; 2^10: 0.028 against 0.026 ms for the integer products),
+// 0.046 ms against 0.057 ms for the best mix of the others; 2^14: 0.121 / 0.167;
+// 2^20: 7.49 / 11.8 ms; 2^10: 0.028 against 0.026 ms for the integer products),
 // so only their splits are timed there.
 constexpr int kTensorMinLog = 12;
 

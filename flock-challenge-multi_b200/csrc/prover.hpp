@@ -75,7 +75,7 @@ struct VerifyStatement {
 // "" when the bundle verifies, otherwise the name of the failed check
 std::string verify_bundle(const uint8_t* bytes, size_t len, const std::string& domain, const VerifyStatement& V);
 
-// A verifier with its own device scratch (8 MiB) and stream, for any
+// A verifier with its own device scratch (9.5 MiB) and stream, for any
 // statement size; the block matrices' device copy is shared per device.  One
 // thread at a time per Verifier.
 class Verifier {

@@ -18,7 +18,8 @@
 // operands' stores and the tensor cores' reads, 56 KiB a step).  Measured at
 // 2^18 / 2^14 / 2^10 compressions: 747 / 54 / 7.4 us, against 1097 / 90 / 20 us
 // for XORs of eq values through 256-entry subset tables (a thread 16 bits of
-// every block).  The same kernel with round 1's group weights took 1262 us for
+// every block); the checks on its waits have since added 3 % at 2^18 (710 to 733
+// us by the profiler's clock).  The same kernel with round 1's group weights took 1262 us for
 // the c column's statistic at 2^18, whose table kernel takes 665 us.
 #include "kernels.cuh"
 #include "tmap.cuh"

@@ -401,7 +401,7 @@ int flock_chain_blocks(uint64_t seed, const uint32_t* initial_cv, size_t steps, 
 int flock_verify(flock_setup* s, const uint8_t* bytes, size_t len, const uint8_t* domain, size_t dlen);
 /* The same verification without a prover setup, for any supported size
  * (2^8..2^20 compressions, read from the bundle): a verifier held by the
- * context and created on first use, with 8 MiB of device scratch, plus
+ * context and created on first use, with 9.5 MiB of device scratch, plus
  * one device copy of the block matrices per device (about 45 MB, kept until
  * the process exits).  Calls on one context are serialised. */
 int flock_verify_bundle(flock_ctx* ctx, const uint8_t* bytes, size_t len, const uint8_t* domain, size_t dlen);
